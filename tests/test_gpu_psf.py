@@ -308,3 +308,64 @@ def test_listmode_osem_with_variant_psf_vs_reference(tmp_path):
     ref, _ = po.ref_osem_listmode(osc, oip, rs[0], e["d1"], e["d2"], iterations=2,
                                   subsets=2, image_psf_csv=csv, image_psf_variant=True)
     assert rel_l2(img, ref) < 1e-4
+
+
+def _varpsf_by_taps(img, kernels, lut, gap, voxel, adjoint):
+    """The operator one tap at a time in FP32 (products and sums rounded
+    separately, taps in z, y, x order): bit for bit applyA's order."""
+    which = []
+    for n, g, m, v in zip(img.shape[:0:-1], gap, lut, voxel):
+        t = np.abs((np.arange(n) + 0.5) * np.float64(np.float32(v)) -
+                   np.float32(np.float32(n) * np.float32(v) / np.float32(2))).astype(np.float32)
+        a = np.floor(t / np.float32(g) + np.float32(0.5)).astype(np.int64)
+        which.append(np.minimum(a, m - 1))
+    k = which[0][None, None] + lut[0] * (which[1][None, :, None] + lut[1] * which[2][:, None, None])
+    out = np.zeros_like(img)
+    for i, w in enumerate(kernels):
+        mine = np.broadcast_to(k == i, img.shape)
+        src = np.where(mine, img, np.float32(0)) if adjoint else img
+        acc = np.zeros_like(img)
+        hz, hy, hx = (s // 2 for s in w.shape)
+        for dz in range(-hz, hz + 1):
+            for dy in range(-hy, hy + 1):
+                for dx in range(-hx, hx + 1):
+                    d = (dz, dy, dx) if adjoint else (-dz, -dy, -dx)
+                    acc += np.roll(src, d, (1, 2, 3)) * w[dz + hz, dy + hy, dx + hx]
+        out += acc if adjoint else np.where(mine, acc, np.float32(0))
+    return out
+
+
+# Tile edges (32 x 32 voxels, chunks of 8), images smaller than a tile, frames,
+# kernels from 1 tap to the register window's widest (17) and one beyond it
+# (the one-voxel-per-thread form), one LUT entry or 3 x 3 x 2, and segments too
+# short for the tiled form.
+@pytest.mark.parametrize("shape,half,gaps", [
+    ((1, 3, 4, 5), (1, 1, 1), 1), ((1, 9, 31, 33), (2, 1, 2), 2), ((2, 10, 37, 70), (4, 2, 3), 2),
+    ((1, 8, 32, 64), (0, 0, 0), 2), ((1, 7, 33, 65), (3, 3, 1), 2), ((1, 5, 20, 41), (8, 2, 1), 2),
+    ((1, 5, 20, 41), (9, 1, 1), 2), ((1, 4, 12, 40), (2, 2, 1), 12),
+])
+def test_varpsf_tiles_vs_taps(shape, half, gaps):
+    nt, nz, ny, nx = shape
+    rng = np.random.default_rng(nx * 31 + half[0])
+    voxel = (2.0, 1.5, 3.0)
+    ip = yrt.ImageParams(nx, ny, nz, nx * 2.0, ny * 1.5, nz * 3.0, nt=nt)
+    lut = (gaps + 1, gaps + 1, 2) if gaps > 1 else (1, 1, 1)
+    rg = [0.5 * n * v for n, v in zip((nx, ny, nz), voxel)]
+    gap = [rg[0] / gaps, rg[1] / gaps, rg[2]] if gaps > 1 else [2 * r for r in rg]
+    kernels = []
+    for i in range(lut[0] * lut[1] * lut[2]):
+        h = [int(rng.integers(0, m + 1)) if i else m for m in half]
+        kernels.append(rng.random([2 * h[2] + 1, 2 * h[1] + 1, 2 * h[0] + 1], np.float32))
+    op = yrt.OperatorVarPsfDevice(ip)
+    op.setKernelCollection(kernels)
+    op.setRangeAndGap(rg[0], gap[0], rg[1], gap[1], rg[2], gap[2])
+    img = rng.random(shape, np.float32)
+    x = torch.from_numpy(img).cuda()
+    fwd = op.applyA(x, torch.empty_like(x), ip).cpu().numpy()
+    assert np.array_equal(bits(fwd), bits(_varpsf_by_taps(img, kernels, lut, gap, voxel, False)))
+    adj = op.applyAH(x, torch.empty_like(x), ip).cpu().numpy()
+    want = _varpsf_by_taps(img.astype(np.float64), [k.astype(np.float64) for k in kernels], lut,
+                           gap, voxel, True)
+    # n positive FP32 terms: at most n roundings of half an ulp of the sum.
+    n = int(np.prod([2 * h + 1 for h in half]))
+    assert rel_l2(adj, want) < max(2, n) * 2.0 ** -24

@@ -39,8 +39,9 @@ def _compile(src, out, deps, verbose):
 
 def build(verbose: bool = False) -> str:
     os.makedirs(os.path.dirname(OUT), exist_ok=True)
-    _compile(SRC, OUT, [SRC, os.path.join(HERE, "csrc", "device.cuh"),
-                        os.path.join(ROOT, "include", "yrt_b200.h")], verbose)
+    csrc = os.path.join(HERE, "csrc")
+    headers = [os.path.join(csrc, f) for f in sorted(os.listdir(csrc)) if f.endswith(".cuh")]
+    _compile(SRC, OUT, [SRC, *headers, os.path.join(ROOT, "include", "yrt_b200.h")], verbose)
     _compile(L2_SRC, L2_OUT, [L2_SRC], verbose)
     return OUT
 

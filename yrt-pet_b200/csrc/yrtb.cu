@@ -23,6 +23,7 @@
 
 #include "yrt_b200.h"
 #include "device.cuh"
+#include "varpsf_tile.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
@@ -2093,32 +2094,8 @@ void psfPass(dim3 grid, dim3 block, cudaStream_t st, const float* src, float* ds
 }
 
 // ------------------------------------------- spatially variant image PSF --
-// OperatorVarPsf (src/operators/OperatorVarPsf.cpp:290-455): every voxel has
-// its own 3-D kernel, the LUT entry nearest to |voxel centre - image centre|
-// (x, y, z gaps, clamped at the LUT's range).
-struct VarPsfDev
-{
-	const float* w;     // all kernels' weights, z-major, then y, then x
-	const int4* meta;   // per kernel: offset into w, half sizes x, y, z
-	int lutX, lutY, lutZ;
-	float gapX, gapY, gapZ;
-	float vx, vy, vz;
-	float cx, cy, cz;   // image centre: n * v / 2 in FP32
-	int maxHx, maxHy, maxHz;
-};
-
-// LUT coordinate of index i along one axis (OperatorVarPsf::findNearestKernel
-// with the distances of varconvolve: |(i + 0.5) v - centre| in FP64, then
-// FP32, divided by the gap, rounded, clamped).  The LUT index of voxel
-// (i, j, k) is a(i) + A (b(j) + B c(k)): separable, so each block tabulates
-// the three axes once in shared memory.
-__device__ __forceinline__ int varPsfAxis(int i, float v, float centre, float gap, int dim)
-{
-	const float t = static_cast<float>(fabs((i + 0.5) * static_cast<double>(v) - centre));
-	const int a = static_cast<int>(roundf(fabsf(t) / gap));
-	return a >= dim ? dim - 1 : a;
-}
-
+// One voxel per thread, for LUTs and kernels outside the tiled form's range
+// (varpsf_tile.cuh).
 __device__ __forceinline__ int circ1(int n, int x)
 {
 	return x < 0 ? x + n : (x >= n ? x - n : x);
@@ -2582,6 +2559,9 @@ struct yrtb_varpsf
 {
 	float* w = nullptr;
 	int4* meta = nullptr;
+	// The same kernels with their rows padded to 4 floats (tiled form).
+	float4* wRows = nullptr;
+	int4* metaRows = nullptr;
 	int numKernels = 0;
 	int lut[3] = {0, 0, 0};
 	float gap[3] = {0, 0, 0};
@@ -2591,6 +2571,8 @@ struct yrtb_varpsf
 	{
 		cudaFree(w);
 		cudaFree(meta);
+		cudaFree(wRows);
+		cudaFree(metaRows);
 	}
 };
 
@@ -4566,8 +4548,102 @@ yrtb_status yrtb_varpsf_create(const float* weights, const int32_t* half_sizes,
 	YRTB_CUDA(cudaMemcpy(p->w, weights, total * sizeof(float), cudaMemcpyHostToDevice));
 	YRTB_CUDA(cudaMemcpy(p->meta, meta.data(), num_kernels * sizeof(int4),
 	                     cudaMemcpyHostToDevice));
+	if (p->maxH[0] <= kVarMaxHx &&
+	    std::all_of(weights, weights + total, [](float k) { return std::isfinite(k); }))
+	{
+		std::vector<float> rows;
+		std::vector<int4> metaRows(num_kernels);
+		for (int i = 0; i < num_kernels; i++)
+		{
+			const int nt = 2 * meta[i].y + 1;
+			metaRows[i] = meta[i];
+			metaRows[i].x = static_cast<int>(rows.size() / 4);
+			const float* k = weights + meta[i].x;
+			for (int r = 0; r < (2 * meta[i].z + 1) * (2 * meta[i].w + 1); r++, k += nt)
+			{
+				rows.insert(rows.end(), k, k + nt);
+				rows.resize((rows.size() + 3) / 4 * 4, 0.f);
+			}
+		}
+		YRTB_CUDA(cudaMalloc(&p->wRows, rows.size() * sizeof(float)));
+		YRTB_CUDA(cudaMalloc(&p->metaRows, num_kernels * sizeof(int4)));
+		YRTB_CUDA(cudaMemcpy(p->wRows, rows.data(), rows.size() * sizeof(float),
+		                     cudaMemcpyHostToDevice));
+		YRTB_CUDA(cudaMemcpy(p->metaRows, metaRows.data(), num_kernels * sizeof(int4),
+		                     cudaMemcpyHostToDevice));
+	}
 	*out = p.release();
 	return YRTB_OK;
+}
+
+// Launch parameters of the tiled variant PSF; false where the one-voxel-per-
+// thread form is used instead: kernels wider than the register window or not finite, a LUT
+// so fine along x that a chunk of 8 outputs would rarely be whole (segments
+// of 8 voxels on average, at most kVarMaxSeg of them), or a halo that leaves
+// no room for two blocks of the smallest tile per SM (113 KB each).
+static bool varTileFits(const yrtb_varpsf* p, const VarPsfDev& P, const int* dims, int64_t nt,
+                        bool adjoint, VarTile& T)
+{
+	if (!p->wRows)
+		return false;
+	T.w = p->wRows;
+	T.meta = p->metaRows;
+	T.Hx = p->maxH[0];
+	T.Hy = p->maxH[1];
+	T.Hz = p->maxH[2];
+	const int H[3] = {T.Hx, T.Hy, T.Hz}, lut[3] = {P.lutX, P.lutY, P.lutZ};
+	const float v[3] = {P.vx, P.vy, P.vz}, c[3] = {P.cx, P.cy, P.cz};
+	const float gap[3] = {P.gapX, P.gapY, P.gapZ};
+	VarSegs* S[3] = {&T.x, &T.y, &T.z};
+	for (int a = 0, stride = 1; a < 3; stride *= lut[a++])
+	{
+		const int n = dims[a];
+		// The forward chunks of x cover the image itself.
+		const int lo = a == 0 && !adjoint ? 0 : -H[a], hi = a == 0 && !adjoint ? n : n + H[a];
+		if (hi > 32767)
+			return false;
+		int last = -1;
+		S[a]->n = 0;
+		for (int i = lo; i < hi; i++)
+		{
+			const int k = varPsfAxis((i + n) % n, v[a], c[a], gap[a], lut[a]);
+			if (k == last)
+				continue;
+			if (S[a]->n == kVarMaxSeg)
+				return false;
+			last = k;
+			S[a]->lut[S[a]->n] = k * stride;
+			S[a]->start[S[a]->n++] = static_cast<short>(i);
+		}
+		S[a]->start[S[a]->n] = static_cast<short>(hi);
+	}
+	const int nx = dims[0];
+	if (T.x.n > 1 && T.x.n * kVarOut > nx)
+		return false;
+	T.chunks = (nx + kVarOut - 1) / kVarOut;
+	if (!adjoint)
+	{
+		T.chunkBase[0] = 0;
+		for (int s = 0; s < T.x.n; s++)
+			T.chunkBase[s + 1] = static_cast<short>(
+			    T.chunkBase[s] + (T.x.start[s + 1] - T.x.start[s] + kVarOut - 1) / kVarOut);
+		T.chunks = T.chunkBase[T.x.n];
+	}
+	// Planes per tile: 8 (3 reads per voxel with a halo of 4) unless that
+	// leaves SMs without a block, at least 2 (8 warps, 4 chunks per plane).
+	const int64_t cols = static_cast<int64_t>((T.chunks + 3) / 4) *
+	                     ((dims[1] + kVarTileY - 1) / kVarTileY);
+	constexpr size_t kTwoPerSM = 113 * 1024;
+	for (T.zt = 8;; T.zt /= 2)
+	{
+		T.zTiles = (dims[2] + T.zt - 1) / T.zt;
+		const int64_t blocks = cols * T.zTiles * nt;
+		if (varShared(T) <= kTwoPerSM &&
+		    (T.zt == 2 || blocks >= 4 * static_cast<int64_t>(gridFor(1u << 30, 1))))
+			return T.zTiles * nt <= 65535;
+		if (T.zt == 2)
+			return false;
+	}
 }
 
 void yrtb_varpsf_destroy(yrtb_varpsf* p)
@@ -4591,6 +4667,9 @@ yrtb_status yrtb_varpsf_apply(const yrtb_varpsf* p, const float* d_in, float* d_
 	if ((dims[1] + kPsfBY - 1) / kPsfBY > 65535 ||
 	    static_cast<int64_t>(ip->nz) * ip->nt > INT32_MAX)
 		return fail(YRTB_ERR_ARGUMENT, "image too large for the PSF launch");
+	const size_t smem = static_cast<size_t>(dims[0] + dims[1] + dims[2]) * sizeof(int);
+	if (smem > 48 * 1024)
+		return fail(YRTB_ERR_ARGUMENT, "image too large for the variant PSF (nx + ny + nz > 12288)");
 	YRTB_CUDA(cudaSetDevice(p->device));
 	VarPsfDev P;
 	P.w = p->w;
@@ -4610,6 +4689,24 @@ yrtb_status yrtb_varpsf_apply(const yrtb_varpsf* p, const float* d_in, float* d_
 	P.maxHx = p->maxH[0];
 	P.maxHy = p->maxH[1];
 	P.maxHz = p->maxH[2];
+	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+	VarTile T;
+	if (varTileFits(p, P, dims, ip->nt, adjoint != 0, T))
+	{
+		const size_t shared = varShared(T);
+		const dim3 tiles((T.chunks + kVarTileX / kVarOut - 1) / (kVarTileX / kVarOut),
+		                 (dims[1] + kVarTileY - 1) / kVarTileY,
+		                 static_cast<unsigned>(T.zTiles * ip->nt));
+		auto go = [&](auto kernel) -> yrtb_status
+		{
+			YRTB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			                               static_cast<int>(shared)));
+			kernel<<<tiles, kVarThreads, shared, st>>>(d_in, d_out, dims[0], dims[1], dims[2], T);
+			YRTB_LAUNCHED();
+			return YRTB_OK;
+		};
+		return adjoint ? go(k_varpsf_tile<true>) : go(k_varpsf_tile<false>);
+	}
 	const int planes = static_cast<int>(ip->nz * ip->nt);
 	const dim3 block(kPsfBX, kPsfBY);
 	// Enough blocks for a few waves; each loops over planes so that the
@@ -4618,10 +4715,6 @@ yrtb_status yrtb_varpsf_apply(const yrtb_varpsf* p, const float* d_in, float* d_
 	const int want = static_cast<int>(gridFor(1u << 30, 16));
 	const int gz = std::max(1, std::min(planes, (want + gx * gy - 1) / (gx * gy)));
 	const dim3 grid(gx, gy, std::min(gz, 65535));
-	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-	const size_t smem = static_cast<size_t>(dims[0] + dims[1] + dims[2]) * sizeof(int);
-	if (smem > 48 * 1024)
-		return fail(YRTB_ERR_ARGUMENT, "image too large for the variant PSF (nx + ny + nz > 12288)");
 	if (adjoint)
 		k_varpsf<true><<<grid, block, smem, st>>>(d_in, d_out, dims[0], dims[1], dims[2], planes, P);
 	else
