@@ -209,3 +209,18 @@ def test_lrem_update_h_vs_reference():
     assert np.array_equal(bits(W_ref.reshape(R, -1)), bits(expect_W))
     assert not np.allclose(H, H0)
     assert rel_l2(H, H_ref) < 1e-4
+
+
+# Tiles of 4 x 4 pairs: one pair, a ragged tile each way, the most tiles
+# (one voxel group each), the largest rank; fewer voxels than groups.
+@pytest.mark.parametrize("R,T,J", [(1, 1, 3), (5, 6, 1), (6, 20, 12345), (5, 409, 300),
+                                   (32, 64, 513), (4, 4, 129), (1, 439, 130)])
+def test_contract_h_pair_tiles(R, T, J):
+    rng = np.random.default_rng(R * 1000 + T)
+    W = rng.standard_normal((R, J)).astype(np.float32)
+    E = rng.standard_normal((T, J)).astype(np.float32)
+    got = lrem.lr_contract_h(torch.from_numpy(W).cuda(), torch.from_numpy(E).cuda(), R)
+    want = W.astype(np.float64) @ E.astype(np.float64).T
+    # Exact products, at most J FP64 roundings of partial sums of |w||e|.
+    bound = J * 2.0 ** -52 * (np.abs(W).astype(np.float64) @ np.abs(E).astype(np.float64).T)
+    assert np.all(np.abs(got.cpu().numpy() - want) <= bound + 1e-300)
