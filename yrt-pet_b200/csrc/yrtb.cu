@@ -595,6 +595,8 @@ __device__ __forceinline__ void redV2(float* p, float2 v)
 // instead of groups of four, held in registers and sent as one
 // red.global.add.v2.f32 (more requests than VEC 1, fewer instructions per
 // visit).
+// The last group of an image whose size is no multiple of 4 (or the last pair
+// of an odd one) is sent voxel by voxel: whole groups are those below `whole`.
 template <int KIND, bool TOF, bool COMP, bool FIX = false, int VEC = 0,
           bool TILE = false>
 __device__ __forceinline__ void backwardEvent(const KParams& P,
@@ -628,11 +630,16 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
 		static_assert(KIND == K_SIDDON || KIND == K_SIDDON_MR,
 		              "slots hold one value per voxel of one ray");
 		int gb = -1;
+		const unsigned size = static_cast<unsigned>(P.g.nvox), whole = size & ~3u;
 		auto send = [&]
 		{
 			const float4 a = make_float4(vslot[0], vslot[vstride], vslot[2 * vstride],
 			                             vslot[3 * vstride]);
-			redV4(img + gb, a);
+			if (static_cast<unsigned>(gb) < whole)
+				redV4(img + gb, a);
+			else
+				for (unsigned l = 0; gb + l < size; l++)
+					atomicAdd(img + gb + l, vslot[l * vstride]);
 		};
 		auto visit = [&](int o, float w)
 		{
@@ -664,13 +671,30 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
 		              "lanes hold one value per voxel of one ray");
 		int gb = -1;
 		float4 a4 = make_float4(0.f, 0.f, 0.f, 0.f);
+		// No group in hand (gb = -1) compares above `whole` too.
+		const unsigned size = static_cast<unsigned>(P.g.nvox), whole = size & ~3u;
+		auto send = [&]
+		{
+			if (static_cast<unsigned>(gb) < whole)
+			{
+				redV4(img + gb, a4);
+			}
+			else if (gb >= 0)
+			{
+				atomicAdd(img + gb, a4.x);
+				if (gb + 1 < size)
+					atomicAdd(img + gb + 1, a4.y);
+				if (gb + 2 < size)
+					atomicAdd(img + gb + 2, a4.z);
+			}
+		};
 		auto visit = [&](int o, float w)
 		{
 			const float c = v * w;
 			const int g = o & ~3;
 			const bool nw = g != gb;
-			if (nw && gb >= 0)
-				redV4(img + gb, a4);
+			if (nw)
+				send();
 			gb = g;
 			// A single-ray walk visits each voxel once: a lane is set, never
 			// summed, inside a group (and cleared when a new group starts).
@@ -682,8 +706,7 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
 		};
 		auto flush = [&]
 		{
-			if (gb >= 0)
-				redV4(img + gb, a4);
+			send();
 			gb = -1;
 		};
 		projectEvent<KIND, TOF, COMP, TILE>(P, p1, p2, n1, n2, tofv, rid, false, visit,
@@ -695,13 +718,21 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
 		              "lanes hold one value per voxel of one ray");
 		int gb = -1;
 		float2 a2 = make_float2(0.f, 0.f);
+		const unsigned whole = static_cast<unsigned>(P.g.nvox) & ~1u;
+		auto send = [&]
+		{
+			if (static_cast<unsigned>(gb) < whole)
+				redV2(img + gb, a2);
+			else if (gb >= 0)
+				atomicAdd(img + gb, a2.x);
+		};
 		auto visit = [&](int o, float w)
 		{
 			const float c = v * w;
 			const int g = o & ~1;
 			const bool nw = g != gb;
-			if (nw && gb >= 0)
-				redV2(img + gb, a2);
+			if (nw)
+				send();
 			gb = g;
 			// Set, never summed, inside a pair (cleared when a new one starts).
 			const bool hi = (o & 1) != 0;
@@ -710,8 +741,7 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
 		};
 		auto flush = [&]
 		{
-			if (gb >= 0)
-				redV2(img + gb, a2);
+			send();
 			gb = -1;
 		};
 		projectEvent<KIND, TOF, COMP, TILE>(P, p1, p2, n1, n2, tofv, rid, false, visit,
@@ -2755,12 +2785,14 @@ void launchTuned(const yrtb_projector* h, const Events& E, Range R,
                  const float* in, float* out, float gs, float thr,
                  cudaStream_t st, const Fixed& F)
 {
-	// Float4 groups need 16-byte aligned frames of the images read and
-	// written (every frame starts at a multiple of nvox floats).
+	// Float4 groups need a 16-byte aligned image, and with several frames
+	// (each starts at a multiple of nvox floats) a multiple of 4 voxels; float4
+	// gathers also need a whole last group (reductions send it voxel by voxel).
 	const float* img = OP == OP_BWD ? out : in;
-	const bool aligned = (reinterpret_cast<uintptr_t>(img) % 16 == 0) &&
-	                     (OP != OP_EM || reinterpret_cast<uintptr_t>(out) % 16 == 0) &&
-	                     (h->P.g.nvox % 4 == 0);
+	const bool base = (reinterpret_cast<uintptr_t>(img) % 16 == 0) &&
+	                  (OP != OP_EM || reinterpret_cast<uintptr_t>(out) % 16 == 0);
+	const bool quads = h->P.g.nvox % 4 == 0;
+	const bool aligned = base && (quads || h->ip.nt == 1);
 	auto go = [&](auto tplc)
 	{
 		constexpr int TPL = decltype(tplc)::value;
@@ -2776,6 +2808,8 @@ void launchTuned(const yrtb_projector* h, const Events& E, Range R,
 			constexpr int kUse = K == K_SIDDON_MR ? (OP == OP_FWD ? 0 : 10)
 			                                      : (OP == OP_FWD ? 1 : (OP == OP_BWD ? 14 : 15));
 			int vg = aligned ? (h->launch.vector_groups & kUse) : 0;
+			if (!quads)
+				vg &= ~1;
 			if (vg & 4)
 				vg &= ~2;
 			if (vg & 6)
