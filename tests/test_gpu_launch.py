@@ -202,3 +202,32 @@ def test_release_cached_memory_after_ordering():
     yrt.release_cached_memory()
     out2, offs2 = p.order_events(ev, 2)   # the pool grows again on demand
     assert torch.equal(out.perm, out2.perm)
+
+
+# Images whose size is no multiple of 4 or 2: the last group of the vector
+# reductions is sent voxel by voxel.  nx = 1 puts every ray's last voxels in it.
+@pytest.mark.parametrize("precision", [L.YRTB_MIRROR, L.YRTB_COMPENSATED])
+@pytest.mark.parametrize("dims", [(61, 63, 31), (30, 31, 15), (1, 1, 3), (1, 5, 1), (2, 3, 1)])
+def test_vector_reductions_on_ragged_images(precision, dims):
+    sc = yrt.Scanner("t", *SC_ARGS)
+    ip = yrt.ImageParams(*dims, 128, 128, 64)
+    pp = yrt.ProjectorParams(sc)
+    pp.precision = precision
+    p = yrt.DeviceProjector(sc, ip, pp)
+    d1, d2 = random_events(20000, 51)
+    ev = yrt.DeviceEvents.from_arrays(d1, d2)
+    y = torch.rand(len(d1), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
+    n = ip.numVoxels
+
+    def back(groups):
+        p.set_launch(256, 1, 3, vector_groups=groups)
+        buf = torch.zeros(n + 8, device="cuda")  # torch's allocations are 512-byte aligned
+        p.backward(y, ev, img=buf[:n])
+        assert not buf[n:].any()
+        return buf[:n].cpu().numpy()
+
+    scalar = back(0)
+    for groups in (2, 4, 8):
+        # The same FP32 terms in two orders, at most all of them in one
+        # voxel: half an ulp per addition, at random, on each side.
+        assert rel_l2(back(groups), scalar) < 2 * len(d1) ** 0.5 * 2.0 ** -24
