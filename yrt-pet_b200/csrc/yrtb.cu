@@ -77,29 +77,12 @@ constexpr int kBlock = 256;
 // Integer maps of the reference Histogram3D (Histogram3D.cpp:165-450) in a
 // form a kernel can evaluate: the in-ring pair <-> (r, phi) map becomes a
 // dense dpr x dpr table, the z-bin decode loop becomes a table of (z1, z2).
+// The host keeps the dimensions; the tables are made on the device
+// (k_h3_ring, k_h3_zpairs).
 struct H3Host
 {
 	uint64_t numR, numPhi, numZBin, numZBinDiff, numDOIPoss, rCut;
 	uint64_t dpr, rings, ndoi, mrd;
-	std::vector<int32_t> ringMap;  // d1_ring*dpr + d2_ring -> r_ring*dpr + phi | -1
-	std::vector<int2> zPairs;      // z_bin -> (z1, z2)
-
-	void pairInRing(uint64_t r_ring, uint64_t phi, uint32_t& a, uint32_t& b) const
-	{
-		const int n = static_cast<int>(dpr);
-		const int r = static_cast<int>(r_ring);
-		const int d02 = (phi % 2 != 0) ? n / 2 + 1 : n / 2;
-		int dr1 = r - n / 4 + static_cast<int>(rCut);
-		int dr2 = d02 - (r - n / 4 + static_cast<int>(rCut));
-		if (dr1 < 0)
-			dr1 += n;
-		if (dr2 < 0)
-			dr2 += n;
-		a = static_cast<uint32_t>((dr1 + static_cast<int>(phi) / 2) % n);
-		b = static_cast<uint32_t>((dr2 + static_cast<int>(phi) / 2) % n);
-		if (a > b)
-			std::swap(a, b);
-	}
 
 	explicit H3Host(const yrtb_scanner& s)
 	{
@@ -116,42 +99,6 @@ struct H3Host
 		const uint64_t nz = (mrd + 1) * rings - (mrd * (mrd + 1)) / 2;
 		numZBinDiff = nz - rings;
 		numZBin = nz + numZBinDiff;
-		ringMap.assign(dpr * dpr, -1);
-		for (uint64_t phi = 0; phi < numPhi; phi++)
-			for (uint64_t r = 0; r < numR / numDOIPoss; r++)
-			{
-				uint32_t a, b;
-				pairInRing(r, phi, a, b);
-				ringMap[a * dpr + b] = static_cast<int32_t>(r * dpr + phi);
-			}
-		zPairs.resize(numZBin);
-		for (uint64_t zb = 0; zb < numZBin; zb++)
-		{
-			int z1, z2;
-			if (zb < rings)
-			{
-				z1 = z2 = static_cast<int>(zb);
-			}
-			else
-			{
-				int cur = (static_cast<int>(zb) - static_cast<int>(rings)) %
-				              static_cast<int>(numZBinDiff) +
-				          static_cast<int>(rings);
-				int planes = static_cast<int>(rings);
-				int dz = 0;
-				while (cur - planes >= 0)
-				{
-					cur -= planes;
-					planes -= 1;
-					dz++;
-				}
-				z1 = cur;
-				z2 = z1 + dz;
-				if (zb - rings >= numZBinDiff)
-					std::swap(z1, z2);
-			}
-			zPairs[zb] = make_int2(z1, z2);
-		}
 	}
 };
 
@@ -207,15 +154,12 @@ __device__ __forceinline__ bool h3Bin(const H3Dev& h, uint32_t d1, uint32_t d2,
 	return true;
 }
 
-__device__ __forceinline__ void h3Pair(const H3Dev& h, uint64_t bin,
-                                       uint32_t& d1, uint32_t& d2)
+// Crystal pair (a <= b) inside a ring of bin (r, phi).
+__device__ __forceinline__ void h3PairInRing(const H3Dev& h, uint32_t r, uint32_t phi,
+                                             uint32_t& a, uint32_t& b)
 {
-	const uint64_t z_bin = bin / (h.numPhi * h.numR);
-	const uint64_t rem = bin % (h.numPhi * h.numR);
-	const uint32_t phi = static_cast<uint32_t>(rem / h.numR);
-	const uint32_t r = static_cast<uint32_t>(rem % h.numR);
 	const int n = static_cast<int>(h.dpr);
-	const int rr = static_cast<int>(r / h.numDOIPoss);
+	const int rr = static_cast<int>(r);
 	const int d02 = (phi % 2 != 0) ? n / 2 + 1 : n / 2;
 	int dr1 = rr - n / 4 + static_cast<int>(h.rCut);
 	int dr2 = d02 - (rr - n / 4 + static_cast<int>(h.rCut));
@@ -223,14 +167,25 @@ __device__ __forceinline__ void h3Pair(const H3Dev& h, uint64_t bin,
 		dr1 += n;
 	if (dr2 < 0)
 		dr2 += n;
-	uint32_t a = static_cast<uint32_t>((dr1 + static_cast<int>(phi) / 2) % n);
-	uint32_t b = static_cast<uint32_t>((dr2 + static_cast<int>(phi) / 2) % n);
+	a = static_cast<uint32_t>((dr1 + static_cast<int>(phi) / 2) % n);
+	b = static_cast<uint32_t>((dr2 + static_cast<int>(phi) / 2) % n);
 	if (a > b)
 	{
 		const uint32_t t = a;
 		a = b;
 		b = t;
 	}
+}
+
+__device__ __forceinline__ void h3Pair(const H3Dev& h, uint64_t bin,
+                                       uint32_t& d1, uint32_t& d2)
+{
+	const uint64_t z_bin = bin / (h.numPhi * h.numR);
+	const uint64_t rem = bin % (h.numPhi * h.numR);
+	const uint32_t phi = static_cast<uint32_t>(rem / h.numR);
+	const uint32_t r = static_cast<uint32_t>(rem % h.numR);
+	uint32_t a, b;
+	h3PairInRing(h, r / h.numDOIPoss, phi, a, b);
 	if (a == b)
 	{
 		d1 = d2 = 0;
@@ -256,6 +211,73 @@ __device__ __forceinline__ uint64_t h3SubsetBin(const H3Dev& h, uint64_t idx,
 	const uint64_t phi = (rem / h.numR) * numSubsets + subset;
 	const uint64_t r = rem % h.numR;
 	return z_bin * h.numPhi * h.numR + phi * h.numR + r;
+}
+
+// Ring map in two passes (map set to -1 before): where several (r, phi) share
+// a pair (a == b), the one with the largest phi, then the largest r, keeps it,
+// whatever order the threads run in; then the entries become r * dpr + phi.
+// A 672-crystal ring takes 225k entries, 4 ms of divisions on the host.
+__global__ void k_h3_ring(H3Dev H, uint32_t ringR, int32_t* __restrict__ map)
+{
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= ringR * H.dpr)
+		return;
+	uint32_t a, b;
+	h3PairInRing(H, i % ringR, i / ringR, a, b);
+	atomicMax(map + static_cast<uint64_t>(a) * H.dpr + b, static_cast<int32_t>(i));
+}
+
+__global__ void k_h3_ring_finish(uint32_t dpr, uint32_t ringR, int32_t* __restrict__ map)
+{
+	const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+	if (i >= static_cast<uint64_t>(dpr) * dpr || map[i] < 0)
+		return;
+	const uint32_t m = static_cast<uint32_t>(map[i]);
+	map[i] = static_cast<int32_t>((m % ringR) * dpr + m / ringR);
+}
+
+// Rings (z1, z2) of each z bin: bins below `rings` are the direct planes, then
+// the ring differences in order, then the same with the rings swapped.
+__global__ void k_h3_zpairs(int rings, int numZBin, int numZBinDiff, int2* __restrict__ zPairs)
+{
+	const int zb = blockIdx.x * blockDim.x + threadIdx.x;
+	if (zb >= numZBin)
+		return;
+	int z1 = zb, z2 = zb;
+	if (zb >= rings)
+	{
+		int cur = (zb - rings) % numZBinDiff + rings;
+		int planes = rings, dz = 0;
+		while (cur - planes >= 0)
+		{
+			cur -= planes;
+			planes -= 1;
+			dz++;
+		}
+		z1 = cur;
+		z2 = z1 + dz;
+		if (zb - rings >= numZBinDiff)
+		{
+			z1 = z2;
+			z2 = cur;
+		}
+	}
+	zPairs[zb] = make_int2(z1, z2);
+}
+
+// Crystal table of a regular cylinder from its in-plane positions and
+// orientations (one per layer and crystal of a ring: x, y, ox, oy) and the
+// rings' z.
+__global__ void k_regular_lut(const float4* __restrict__ cells, const float* __restrict__ z,
+                              uint32_t dpr, uint32_t rings, uint32_t nd,
+                              float4* __restrict__ pos, float4* __restrict__ ori)
+{
+	const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
+	if (d >= nd)
+		return;
+	const float4 c = __ldg(cells + d / (dpr * rings) * dpr + d % dpr);
+	pos[d] = make_float4(c.x, c.y, __ldg(z + d / dpr % rings), 0.f);
+	ori[d] = make_float4(c.z, c.w, 0.f, 0.f);
 }
 
 uint64_t h3SubsetSize(const H3Host& h, uint64_t numSubsets, uint64_t subset,
@@ -1646,23 +1668,37 @@ __global__ void k_gather(const T* __restrict__ in, const unsigned long long* __r
 	}
 }
 
-__global__ void k_multiray_offsets(uint64_t count, int numRays,
-                                   float* __restrict__ out)
+// Each thread takes kMrItems consecutive items: deriving the generator of
+// item k from the seed multiplies the state by about 1.5 skip matrices per two
+// bits of k, from item k - 1 by one.  500,000 items, 3 extra rays: 0.90 ms with
+// a derivation per item.
+constexpr int kMrItems = 8;
+__global__ void __launch_bounds__(kBlock)
+    k_multiray_offsets(uint64_t count, int numRays, float* __restrict__ out)
 {
-	// One item per thread: a warp's threads stay converged across items
-	// (a grid-stride loop lets them drift apart between items).
-	const uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-	const int per = 4 * (numRays - 1);
-	if (k < count)
+	const uint64_t k0 = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * kMrItems;
+	if (k0 >= count)
+		return;
+	MultiRay mr;
+	mr.init(k0, make_float3(1.f, 0.f, 0.f), make_float3(1.f, 0.f, 0.f));
+	curandState base = mr.state;
+	for (uint64_t k = k0; k < k0 + kMrItems && k < count; k++)
 	{
-		MultiRay mr;
-		mr.init(k, make_float3(1.f, 0.f, 0.f), make_float3(1.f, 0.f, 0.f));
-		for (int r = 1; r < numRays; r++)
+		if (k > k0)
+		{
+			skipahead_sequence(1ULL, &base);
+			mr.state = base;
+		}
+		float* row = out + k * 4 * (numRays - 1);
+		for (int r = 1; r < numRays; r++, row += 4)
 		{
 			float u[4];
 			mr.next(u);
-			for (int i = 0; i < 4; i++)
-				out[k * per + 4 * (r - 1) + i] = u[i];
+			if (reinterpret_cast<uintptr_t>(row) % 16 == 0)
+				*reinterpret_cast<float4*>(row) = make_float4(u[0], u[1], u[2], u[3]);
+			else
+				for (int i = 0; i < 4; i++)
+					row[i] = u[i];
 		}
 	}
 }
@@ -2599,20 +2635,43 @@ struct yrtb_projector
 	unsigned* d_fixMax = nullptr;
 	int device = 0;
 
+	// Tables of at most kPooledBytes come from the library's pool (no driver
+	// allocation per projector), larger ones from cudaMalloc.
+	static constexpr size_t kPooledBytes = size_t(64) << 20;
+	std::vector<void*> pooled, owned;
+
+	template <typename T>
+	cudaError_t make(T** p, size_t count)
+	{
+		const size_t bytes = std::max<size_t>(1, count * sizeof(T));
+		const bool pool = bytes <= kPooledBytes;
+		const cudaError_t e = pool ? poolAlloc(p, bytes, nullptr)
+		                           : cudaMalloc(reinterpret_cast<void**>(p), bytes);
+		if (e == cudaSuccess)
+			(pool ? pooled : owned).push_back(*p);
+		return e;
+	}
+
 	~yrtb_projector()
 	{
-		cudaFree(d_fix);
-		cudaFree(d_fixMax);
-		cudaFree(d_pos);
-		cudaFree(d_ori);
-		cudaFree(d_taps);
-		cudaFree(d_flipped);
-		cudaFree(d_prefix);
-		cudaFree(d_prefixFlipped);
-		cudaFree(d_ring);
-		cudaFree(d_z);
-		cudaFree(d_err);
-		cudaFree(d_mrTable);
+		int cur = device;
+		cudaGetDevice(&cur);
+		if (cur != device)
+			cudaSetDevice(device);
+		// Launches on any stream may still read the tables.  Where the wait is
+		// refused (a stream of this thread is being captured) the pooled ones
+		// stay allocated.
+		if (cudaDeviceSynchronize() == cudaSuccess)
+		{
+			for (void* p : pooled)
+				cudaFreeAsync(p, nullptr);
+			if (d_mrTable)
+				cudaFreeAsync(d_mrTable, nullptr);
+		}
+		for (void* p : owned)
+			cudaFree(p);
+		if (cur != device)
+			cudaSetDevice(cur);
 	}
 };
 
@@ -3187,6 +3246,46 @@ yrtb_status scannerCheck(const yrtb_scanner* s)
 	return YRTB_OK;
 }
 
+// DetRegular::generateLUT (DetRegular.cpp:113-183), float arithmetic with the
+// reference's double constants.  The in-plane part does not depend on the
+// ring, so it is computed once per layer and crystal of a ring (x, y and
+// orientation x, y); z[ring] is the rings' position.
+void regularCells(const yrtb_scanner& s, std::vector<float4>& cells, std::vector<float>& z)
+{
+	const double PI_ = 3.14159265358979;
+	const double TWOPI_ = 6.28318530717959;
+	const size_t numBlocks = s.dets_per_ring / s.dets_per_block;
+	const float blockLength = s.crystal_size_trans * s.dets_per_block;
+	cells.resize(s.num_doi * s.dets_per_ring);
+	z.resize(s.num_rings);
+	for (size_t ring = 0; ring < s.num_rings; ring++)
+	{
+		const float zGap = s.axial_fov / static_cast<float>(s.num_rings);
+		z[ring] = -s.axial_fov / 2.0 + (ring + 0.5f) * zGap;
+	}
+	for (size_t doi = 0; doi < s.num_doi; doi++)
+	{
+		const float blockDistance = s.scanner_radius + s.crystal_depth * doi;
+		for (size_t block = 0; block < numBlocks; block++)
+		{
+			const float angle = block * TWOPI_ / numBlocks;
+			const float xb = (blockDistance + 0.5f * s.crystal_depth) * std::cos(angle);
+			const float yb = (blockDistance + 0.5f * s.crystal_depth) * std::sin(angle);
+			for (size_t det = 0; det < s.dets_per_block; det++)
+			{
+				float rel = 0.0f;
+				if (s.dets_per_block != 1)
+					rel = -0.5 + (det + 0.5) / static_cast<float>(s.dets_per_block);
+				const float rx = rel * std::cos(angle + PI_ / 2.0);
+				const float ry = rel * std::sin(angle + PI_ / 2.0);
+				cells[doi * s.dets_per_ring + block * s.dets_per_block + det] =
+				    make_float4(xb + blockLength * rx, yb + blockLength * ry, std::cos(angle),
+				                std::sin(angle));
+			}
+		}
+	}
+}
+
 }  // namespace
 
 // ================================================================ C ABI ===
@@ -3209,44 +3308,18 @@ yrtb_status yrtb_scanner_regular_lut(const yrtb_scanner* s, float* out)
 		return st;
 	if (!out)
 		return fail(YRTB_ERR_ARGUMENT, "null output");
-	// DetRegular::generateLUT (DetRegular.cpp:113-183), float arithmetic with
-	// the reference's double constants.
-	const double PI_ = 3.14159265358979;
-	const double TWOPI_ = 6.28318530717959;
-	const size_t numBlocks = s->dets_per_ring / s->dets_per_block;
-	const float blockLength = s->crystal_size_trans * s->dets_per_block;
+	std::vector<float4> cells;
+	std::vector<float> z;
+	regularCells(*s, cells, z);
+	size_t idx = 0;
 	for (size_t doi = 0; doi < s->num_doi; doi++)
-	{
-		const float blockDistance = s->scanner_radius + s->crystal_depth * doi;
 		for (size_t ring = 0; ring < s->num_rings; ring++)
-		{
-			const float zGap = s->axial_fov / static_cast<float>(s->num_rings);
-			const float zPos = -s->axial_fov / 2.0 + (ring + 0.5f) * zGap;
-			for (size_t block = 0; block < numBlocks; block++)
+			for (size_t d = 0; d < s->dets_per_ring; d++, idx++)
 			{
-				const float angle = block * TWOPI_ / numBlocks;
-				const float xb = (blockDistance + 0.5f * s->crystal_depth) * std::cos(angle);
-				const float yb = (blockDistance + 0.5f * s->crystal_depth) * std::sin(angle);
-				for (size_t det = 0; det < s->dets_per_block; det++)
-				{
-					float rel = 0.0f;
-					if (s->dets_per_block != 1)
-						rel = -0.5 + (det + 0.5) / static_cast<float>(s->dets_per_block);
-					const float rx = rel * std::cos(angle + PI_ / 2.0);
-					const float ry = rel * std::sin(angle + PI_ / 2.0);
-					const size_t idx = det + block * s->dets_per_block +
-					                   ring * s->dets_per_ring +
-					                   doi * (s->num_rings * s->dets_per_ring);
-					out[idx * 6 + 0] = xb + blockLength * rx;
-					out[idx * 6 + 1] = yb + blockLength * ry;
-					out[idx * 6 + 2] = zPos;
-					out[idx * 6 + 3] = std::cos(angle);
-					out[idx * 6 + 4] = std::sin(angle);
-					out[idx * 6 + 5] = 0.0f;
-				}
+				const float4 c = cells[doi * s->dets_per_ring + d];
+				const float row[6] = {c.x, c.y, z[ring], c.z, c.w, 0.0f};
+				std::memcpy(out + idx * 6, row, sizeof(row));
 			}
-		}
-	}
 	return YRTB_OK;
 }
 
@@ -3296,23 +3369,40 @@ yrtb_status yrtb_projector_create(const yrtb_scanner* s, const float* lut,
 	h->pp.psf_taps = nullptr;
 	cudaGetDevice(&h->device);
 	const uint64_t nd = s->dets_per_ring * s->num_rings * s->num_doi;
-	std::vector<float> hl(nd * 6);
-	if (lut)
-		std::memcpy(hl.data(), lut, nd * 6 * sizeof(float));
-	else
-		yrtb_scanner_regular_lut(s, hl.data());
-	std::vector<float4> pos(nd), ori(nd);
-	for (uint64_t d = 0; d < nd; d++)
-	{
-		pos[d] = make_float4(hl[d * 6 + 0], hl[d * 6 + 1], hl[d * 6 + 2], 0.f);
-		ori[d] = make_float4(hl[d * 6 + 3], hl[d * 6 + 4], hl[d * 6 + 5], 0.f);
-	}
-	YRTB_CUDA(cudaMalloc(&h->d_pos, nd * sizeof(float4)));
-	YRTB_CUDA(cudaMalloc(&h->d_ori, nd * sizeof(float4)));
-	YRTB_CUDA(cudaMemcpy(h->d_pos, pos.data(), nd * sizeof(float4), cudaMemcpyHostToDevice));
-	YRTB_CUDA(cudaMemcpy(h->d_ori, ori.data(), nd * sizeof(float4), cudaMemcpyHostToDevice));
-	YRTB_CUDA(cudaMalloc(&h->d_err, sizeof(unsigned long long)));
+	YRTB_CUDA(h->make(&h->d_pos, nd));
+	YRTB_CUDA(h->make(&h->d_ori, nd));
+	YRTB_CUDA(h->make(&h->d_err, 1));
 	YRTB_CUDA(cudaMemset(h->d_err, 0, sizeof(unsigned long long)));
+	if (lut)
+	{
+		std::vector<float4> pos(nd), ori(nd);
+		for (uint64_t d = 0; d < nd; d++)
+		{
+			pos[d] = make_float4(lut[d * 6 + 0], lut[d * 6 + 1], lut[d * 6 + 2], 0.f);
+			ori[d] = make_float4(lut[d * 6 + 3], lut[d * 6 + 4], lut[d * 6 + 5], 0.f);
+		}
+		YRTB_CUDA(cudaMemcpy(h->d_pos, pos.data(), nd * sizeof(float4), cudaMemcpyHostToDevice));
+		YRTB_CUDA(cudaMemcpy(h->d_ori, ori.data(), nd * sizeof(float4), cudaMemcpyHostToDevice));
+	}
+	else
+	{
+		// 11 KB instead of 1.7 MB for 80 rings of 672 crystals.
+		std::vector<float4> cells;
+		std::vector<float> z;
+		regularCells(*s, cells, z);
+		const size_t nc = cells.size();
+		cells.resize(nc + (z.size() + 3) / 4);
+		std::memcpy(cells.data() + nc, z.data(), z.size() * sizeof(float));
+		float4* d_cells = nullptr;
+		YRTB_CUDA(h->make(&d_cells, cells.size()));
+		YRTB_CUDA(cudaMemcpy(d_cells, cells.data(), cells.size() * sizeof(float4),
+		                     cudaMemcpyHostToDevice));
+		k_regular_lut<<<gridAll(nd), kBlock>>>(d_cells, reinterpret_cast<float*>(d_cells + nc),
+		                                       static_cast<uint32_t>(s->dets_per_ring),
+		                                       static_cast<uint32_t>(s->num_rings),
+		                                       static_cast<uint32_t>(nd), h->d_pos, h->d_ori);
+		YRTB_LAUNCHED();
+	}
 
 	KParams& P = h->P;
 	P.g = makeGeom(*ip);
@@ -3338,8 +3428,8 @@ yrtb_status yrtb_projector_create(const yrtb_scanner* s, const float* lut,
 	if (h->det)
 	{
 		const uint64_t J = static_cast<uint64_t>(P.g.nvox) * ip->nt;
-		YRTB_CUDA(cudaMalloc(&h->d_fix, J * sizeof(unsigned long long)));
-		YRTB_CUDA(cudaMalloc(&h->d_fixMax, sizeof(unsigned)));
+		YRTB_CUDA(h->make(&h->d_fix, J));
+		YRTB_CUDA(h->make(&h->d_fixMax, 1));
 	}
 	if (pp->projector == YRTB_SIDDON)
 		h->kind = pp->num_rays > 1 ? K_SIDDON_MR : K_SIDDON;
@@ -3361,8 +3451,8 @@ yrtb_status yrtb_projector_create(const yrtb_scanner* s, const float* lut,
 			for (int j = 0; j < pp->psf_size; j++)
 				flipped[i * pp->psf_size + pp->psf_size - 1 - j] =
 				    pp->psf_taps[i * pp->psf_size + j];
-		YRTB_CUDA(cudaMalloc(&h->d_taps, n * sizeof(float)));
-		YRTB_CUDA(cudaMalloc(&h->d_flipped, n * sizeof(float)));
+		YRTB_CUDA(h->make(&h->d_taps, n));
+		YRTB_CUDA(h->make(&h->d_flipped, n));
 		YRTB_CUDA(cudaMemcpy(h->d_taps, pp->psf_taps, n * sizeof(float), cudaMemcpyHostToDevice));
 		YRTB_CUDA(cudaMemcpy(h->d_flipped, flipped.data(), n * sizeof(float), cudaMemcpyHostToDevice));
 		// Prefix sums of the trapezoid bins per kernel row (FP64, stored FP32).
@@ -3387,8 +3477,8 @@ yrtb_status yrtb_projector_create(const yrtb_scanner* s, const float* lut,
 		std::vector<float> taps(pp->psf_taps, pp->psf_taps + n), pre, preF;
 		prefixOf(taps, pre);
 		prefixOf(flipped, preF);
-		YRTB_CUDA(cudaMalloc(&h->d_prefix, pre.size() * sizeof(float)));
-		YRTB_CUDA(cudaMalloc(&h->d_prefixFlipped, preF.size() * sizeof(float)));
+		YRTB_CUDA(h->make(&h->d_prefix, pre.size()));
+		YRTB_CUDA(h->make(&h->d_prefixFlipped, preF.size()));
 		YRTB_CUDA(cudaMemcpy(h->d_prefix, pre.data(), pre.size() * sizeof(float), cudaMemcpyHostToDevice));
 		YRTB_CUDA(cudaMemcpy(h->d_prefixFlipped, preF.data(), preF.size() * sizeof(float), cudaMemcpyHostToDevice));
 		P.psf = Psf{h->d_taps, h->d_flipped, pp->psf_num_s, pp->psf_size,
@@ -3399,16 +3489,31 @@ yrtb_status yrtb_projector_create(const yrtb_scanner* s, const float* lut,
 	{
 		h->h3 = std::make_unique<H3Host>(*s);
 		const H3Host& H = *h->h3;
-		YRTB_CUDA(cudaMalloc(&h->d_ring, H.ringMap.size() * sizeof(int32_t)));
-		YRTB_CUDA(cudaMalloc(&h->d_z, H.zPairs.size() * sizeof(int2)));
-		YRTB_CUDA(cudaMemcpy(h->d_ring, H.ringMap.data(), H.ringMap.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-		YRTB_CUDA(cudaMemcpy(h->d_z, H.zPairs.data(), H.zPairs.size() * sizeof(int2), cudaMemcpyHostToDevice));
+		// numR wraps around when the angle difference leaves no bin.
+		if (s->min_ang_diff > s->dets_per_ring / 2 + 1)
+			return fail(YRTB_ERR_ARGUMENT, "Minimum angle difference leaves no histogram bin");
+		YRTB_CUDA(h->make(&h->d_ring, H.dpr * H.dpr));
+		YRTB_CUDA(h->make(&h->d_z, H.numZBin));
 		h->h3d = H3Dev{static_cast<uint32_t>(nd), h->d_ring, h->d_z, static_cast<uint32_t>(H.dpr),
 		               static_cast<uint32_t>(H.rings), static_cast<uint32_t>(H.ndoi),
 		               static_cast<uint32_t>(H.numDOIPoss), static_cast<uint32_t>(H.rCut),
 		               static_cast<uint32_t>(H.mrd), H.numR, H.numPhi, H.numZBin,
 		               H.numZBinDiff};
+		const uint32_t ringR = static_cast<uint32_t>(H.numR / H.numDOIPoss);
+		YRTB_CUDA(cudaMemsetAsync(h->d_ring, 0xFF, H.dpr * H.dpr * sizeof(int32_t)));
+		if (ringR > 0)
+		{
+			k_h3_ring<<<gridAll(ringR * H.dpr), kBlock>>>(h->h3d, ringR, h->d_ring);
+			k_h3_ring_finish<<<gridAll(H.dpr * H.dpr), kBlock>>>(
+			    static_cast<uint32_t>(H.dpr), ringR, h->d_ring);
+		}
+		k_h3_zpairs<<<gridAll(H.numZBin), kBlock>>>(
+		    static_cast<int>(H.rings), static_cast<int>(H.numZBin),
+		    static_cast<int>(H.numZBinDiff), h->d_z);
+		YRTB_LAUNCHED();
 	}
+	// The tables are read on whatever stream the caller projects on.
+	YRTB_CUDA(cudaStreamSynchronize(nullptr));
 	*out = h.release();
 	return YRTB_OK;
 }
@@ -3535,7 +3640,7 @@ yrtb_status yrtb_multiray_offsets(yrtb_projector* h, uint64_t count,
 	if (h->P.numRays < 2 || count == 0)
 		return YRTB_OK;
 	YRTB_CUDA(cudaSetDevice(h->device));
-	k_multiray_offsets<<<gridAll(count), kBlock, 0,
+	k_multiray_offsets<<<gridAll((count + kMrItems - 1) / kMrItems), kBlock, 0,
 	                     reinterpret_cast<cudaStream_t>(stream)>>>(
 	    count, h->P.numRays, d_out);
 	YRTB_LAUNCHED();
@@ -3551,17 +3656,21 @@ yrtb_status yrtb_multiray_table(yrtb_projector* h, uint64_t count,
 		return YRTB_OK;
 	YRTB_CUDA(cudaSetDevice(h->device));
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-	// Launches already queued may still read the old table.
-	YRTB_CUDA(cudaDeviceSynchronize());
-	h->P.mrTable = nullptr;
-	h->P.mrCount = 0;
-	YRTB_CUDA(cudaFree(h->d_mrTable));
-	h->d_mrTable = nullptr;
-	h->mrCapacity = 0;
+	if (h->d_mrTable)
+	{
+		// Launches already queued may still read the old table.
+		YRTB_CUDA(cudaDeviceSynchronize());
+		h->P.mrTable = nullptr;
+		h->P.mrCount = 0;
+		h->mrCapacity = 0;
+		float* old = h->d_mrTable;
+		h->d_mrTable = nullptr;
+		YRTB_CUDA(cudaFreeAsync(old, st));
+	}
 	const uint64_t per = 4 * static_cast<uint64_t>(h->P.numRays - 1);
-	YRTB_CUDA(cudaMalloc(&h->d_mrTable, count * per * sizeof(float)));
-	k_multiray_offsets<<<gridAll(count), kBlock, 0, st>>>(count, h->P.numRays,
-	                                                       h->d_mrTable);
+	YRTB_CUDA(poolAlloc(&h->d_mrTable, count * per * sizeof(float), st));
+	k_multiray_offsets<<<gridAll((count + kMrItems - 1) / kMrItems), kBlock, 0, st>>>(
+	    count, h->P.numRays, h->d_mrTable);
 	YRTB_LAUNCHED();
 	h->mrCapacity = count;
 	h->P.mrTable = h->d_mrTable;
