@@ -468,6 +468,18 @@ yrtb_status yrtb_events_gather(const yrtb_events* in, const uint64_t* d_perm,
                                const yrtb_events* out, yrtb_stream stream);
 
 /* ----------------------------------------------------- histogram mode --- */
+/* d_values[bin] = A image, and d_image += A^T d_values, over the bins of one
+ * subset of the projector's Histogram3D (phi = subset mod num_subsets);
+ * d_values holds every bin of the histogram, entries outside the subset are
+ * neither written nor read.  Non-TOF projectors; images of several frames
+ * take the first.  The values are those of yrtb_forward / yrtb_backward on
+ * the bins' crystal pairs (OperatorProjectorDevice::applyA / applyAH with a
+ * histogram's bin iterator, src/operators/OperatorProjectorDevice.cu:442-706),
+ * without event arrays. */
+yrtb_status yrtb_forward_histo3d(yrtb_projector* h, const float* d_image, int num_subsets,
+                                 int subset, float* d_values, yrtb_stream stream);
+yrtb_status yrtb_backward_histo3d(yrtb_projector* h, const float* d_values, int num_subsets,
+                                  int subset, float* d_image, yrtb_stream stream);
 /* Sensitivity image over one subset of Histogram3D bins (phi = subset mod
  * num_subsets), non-TOF: d_sens += A^T (sens_bin * acf_bin).  d_sens_histo /
  * d_acf_histo may be NULL (1); d_mu (with mu_params) gives ACFs from an

@@ -15,6 +15,7 @@ import pytest
 import torch  # noqa: F401  (CUDA context for the operator)
 
 import pyyrtpet_b200 as yrt
+from pyyrtpet_b200 import _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -110,3 +111,61 @@ def test_operator_projector_device_reference_signatures(kind):
     assert np.allclose(img.cpu().numpy(), bp, rtol=1e-5, atol=1e-6)
     with pytest.raises(RuntimeError):
         op.applyA(x, data)          # a ProjectionList receives the values
+
+
+# Subsets of one or many phi, a subset with fewer phi than the others, both
+# precisions and every projector; the lists of crystal pairs are the oracle.
+@pytest.mark.parametrize("projector,rays", [("S", 1), ("S", 3), ("DD", 1)])
+@pytest.mark.parametrize("comp,det", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("subsets,subset", [(1, 0), (7, 6), (32, 31)])
+def test_histogram_bins_equal_crystal_pairs(projector, rays, comp, det, subsets, subset):
+    sc = yrt.Scanner("t", 40, 4, 4, 10, 100, 32, 6, 1, 4, 3, 1)
+    ip = yrt.ImageParams(21, 18, 10, 105.0, 90.0, 40.0)
+    pp = yrt.ProjectorParams(sc)
+    pp.setProjector(projector)
+    pp.numRays = rays
+    pp.precision = L.YRTB_COMPENSATED if comp else L.YRTB_MIRROR
+    pp.deterministic = det
+    h = yrt.Histogram3D(sc)
+    it = h.getBinIter(subsets, subset)
+    rng = np.random.default_rng(subsets)
+    x = torch.from_numpy(rng.random(ip.shape, np.float32)).cuda()
+    w = torch.from_numpy(rng.random(h.histoSize, np.float32)).cuda()
+    p = yrt.DeviceProjector(sc, ip, pp)
+    bins = it.indices()
+    ev = yrt.DeviceEvents.from_arrays(*yrt.histo3d_detpairs(sc, bins))
+    idx = torch.from_numpy(bins).cuda()
+    want = torch.full((h.histoSize,), -7.0, device="cuda")
+    want[idx] = p.forward(x, ev)
+    want_img = p.backward(w[idx].contiguous(), ev)
+    op = yrt.OperatorProjectorDevice.create(pp, it, img_params=ip)
+    got = yrt.ProjectionList(h)
+    got.values = torch.full((h.histoSize,), -7.0, device="cuda")
+    op.applyA(x, got)
+    assert torch.equal(got.values, want)
+    img = torch.zeros(ip.shape, device="cuda")
+    got.values = w.clone()
+    op.applyAH(got, img)
+    if det:
+        assert torch.equal(img, want_img)  # fixed-point sums: any order
+    else:
+        # Positive terms in another order: each of the up to n additions
+        # rounds by half an ulp, at random (sqrt(n)) rather than all one way.
+        n = len(bins)
+        assert float((img - want_img).norm() / want_img.norm()) < n ** 0.5 * 2.0 ** -24 + 1e-6
+    assert torch.equal(got.values, w)
+
+
+def test_histogram_bins_refuse_what_crystal_pairs_refuse():
+    sc = yrt.Scanner("t", 40, 4, 4, 10, 100, 32, 6, 1, 4, 3, 1)
+    ip = yrt.ImageParams(8, 8, 4, 80.0, 80.0, 40.0)
+    h = yrt.Histogram3D(sc)
+    pp = yrt.ProjectorParams(sc)
+    pp.addTOF(214.0, 5)
+    op = yrt.OperatorProjectorDevice.create(pp, h.getBinIter(2, 0), img_params=ip)
+    vals = yrt.ProjectionList(h)
+    vals.allocate()
+    with pytest.raises(RuntimeError, match="requires per-event TOF values"):
+        op.applyA(torch.zeros(ip.shape, device="cuda"), vals)
+    with pytest.raises(RuntimeError, match="requires per-event TOF values"):
+        op.applyAH(vals, torch.zeros(ip.shape, device="cuda"))

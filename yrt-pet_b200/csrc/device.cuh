@@ -163,6 +163,50 @@ __device__ __forceinline__ void slabAlpha(R r0, R r1, R p1, R p2, R inv,
 	}
 }
 
+// Parametric interval of a ray inside the FOV cylinder; false if it misses it.
+__device__ __forceinline__ bool cylinderAlpha(const Geom& g, float3 p1, float3 p2, float& t0,
+                                              float& t1)
+{
+	const float A = (p2.x - p1.x) * (p2.x - p1.x) + (p2.y - p1.y) * (p2.y - p1.y);
+	const float B = 2.0f * ((p2.x - p1.x) * p1.x + (p2.y - p1.y) * p1.y);
+	const float C = p1.x * p1.x + p1.y * p1.y - g.fovRadius * g.fovRadius;
+	const float Delta = B * B - 4.0f * A * C;
+	t0 = 0.f;
+	t1 = 1.f;
+	if (A != 0.0f)
+	{
+		if (Delta <= 0.0f)
+			return false;
+		const float sq = sqrtf(Delta);
+		t0 = (-B - sq) / (2.0f * A);
+		t1 = (-B + sq) / (2.0f * A);
+	}
+	return true;
+}
+
+// Whether a (non-TOF) Siddon walk of the ray has anything to visit, up to the
+// rounding of its last segments: the clip of SiddonWalker::begin, with the
+// same values, leaves an interval.
+__device__ __forceinline__ bool crossesGrid(const Geom& g, float3 p1, float3 p2)
+{
+	float t0, t1;
+	if (!cylinderAlpha(g, p1, p2, t0, t1))
+		return false;
+	float amin = fmaxf(0.0f, t0), amax = fminf(1.0f, t1);
+	auto axis = [&](float a, float b, float half)
+	{
+		const float inv = a == b ? 0.0f : 1.0f / (b - a);
+		float lo, hi;
+		slabAlpha<float>(-half, half, a, b, inv, lo, hi);
+		amin = fmaxf(amin, lo);
+		amax = fminf(amax, hi);
+	};
+	axis(p1.x, p2.x, 0.5f * g.lx);
+	axis(p1.y, p2.y, 0.5f * g.ly);
+	axis(p1.z, p2.z, 0.5f * g.lz);
+	return amin < amax;
+}
+
 // ------------------------------------------------------------ Siddon ----
 // Walks one ray through the image grid and calls visit(offset, weight) for
 // each voxel crossing, in order.  p1, p2: endpoints relative to the image
@@ -285,25 +329,8 @@ struct SiddonWalker
 		p2 = q2;
 		// 1. Clip to the FOV cylinder.
 		float t0, t1;
-		{
-			const float A = (p2.x - p1.x) * (p2.x - p1.x) + (p2.y - p1.y) * (p2.y - p1.y);
-			const float B = 2.0f * ((p2.x - p1.x) * p1.x + (p2.y - p1.y) * p1.y);
-			const float C = p1.x * p1.x + p1.y * p1.y - g.fovRadius * g.fovRadius;
-			const float Delta = B * B - 4.0f * A * C;
-			if (A != 0.0f)
-			{
-				if (Delta <= 0.0f)
-					return false;
-				const float sq = sqrtf(Delta);
-				t0 = (-B - sq) / (2.0f * A);
-				t1 = (-B + sq) / (2.0f * A);
-			}
-			else
-			{
-				t0 = 0.f;
-				t1 = 1.f;
-			}
-		}
+		if (!cylinderAlpha(g, p1, p2, t0, t1))
+			return false;
 		const float3 d12 = f3sub(p1, p2);
 		d_norm = sqrtf(d12.x * d12.x + d12.y * d12.y + d12.z * d12.z);
 		const bool flat_x = (p1.x == p2.x);

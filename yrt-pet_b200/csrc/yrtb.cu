@@ -381,16 +381,25 @@ __device__ __forceinline__ bool fetchEvent(const KParams& P, const Events& E,
 
 // Runs the configured projector over one event; endRay() after each ray.
 // TILE: the image is in 4 x 2 tiles (tileOffset; single-ray Siddon only).
-template <int KIND, bool TOF, bool COMP, bool TILE = false, typename Visit, typename EndRay>
+// WARP: all 32 lanes call it and walk in lock step (siddonWalkWarp), lanes with
+// alive == false without a ray (single-ray Siddon only); same visits.
+template <int KIND, bool TOF, bool COMP, bool TILE = false, bool WARP = false,
+          typename Visit, typename EndRay>
 __device__ __forceinline__ void projectEvent(const KParams& P, float3 p1,
                                              float3 p2, float3 n1, float3 n2,
                                              float tofv, uint64_t rid,
                                              bool forward, Visit& visit,
                                              EndRay& endRay, int part = 0,
-                                             int parts = 1)
+                                             int parts = 1, bool alive = true)
 {
 	static_assert(!TILE || KIND == K_SIDDON, "tiled images: single-ray Siddon");
-	if constexpr (KIND == K_SIDDON)
+	static_assert(!WARP || (KIND == K_SIDDON && !TILE), "lock step: single-ray Siddon");
+	if constexpr (WARP)
+	{
+		siddonWalkWarp<TOF, COMP>(alive, P.g, p1, p2, P.tof, tofv, visit);
+		endRay();
+	}
+	else if constexpr (KIND == K_SIDDON)
 	{
 		siddonWalk<TOF, COMP, TILE>(P.g, p1, p2, P.tof, tofv, visit, 0.f, 1.f, part,
 		                            parts);
@@ -472,14 +481,15 @@ __device__ __forceinline__ void projectEvent(const KParams& P, float3 p1,
 // VEC: the image is read as aligned float4 groups, and consecutive
 // crossings inside one group (x steps) reuse the group held in registers.
 template <int KIND, bool TOF, bool COMP, bool TRACK = false, bool VEC = false,
-          bool TILE = false>
+          bool TILE = false, bool WARP = false>
 __device__ __forceinline__ float forwardEvent(const KParams& P,
                                               const float* __restrict__ img,
                                               float3 p1, float3 p2, float3 n1,
                                               float3 n2, float tofv,
                                               uint64_t rid,
                                               float* maxw = nullptr,
-                                              int part = 0, int parts = 1)
+                                              int part = 0, int parts = 1,
+                                              bool alive = true)
 {
 	float acc = 0.f, ray = 0.f, comp = 0.f, mw = 0.f;
 	int gb = -1;
@@ -524,8 +534,8 @@ __device__ __forceinline__ float forwardEvent(const KParams& P,
 		ray = 0.f;
 		comp = 0.f;
 	};
-	projectEvent<KIND, TOF, COMP, TILE>(P, p1, p2, n1, n2, tofv, rid, true, visit,
-	                                    endRay, part, parts);
+	projectEvent<KIND, TOF, COMP, TILE, WARP>(P, p1, p2, n1, n2, tofv, rid, true, visit,
+	                                          endRay, part, parts, alive);
 	// One lane per ray (parts > 1): the caller adds the rays' sums in ray
 	// order and divides (rayGroupMean).
 	if constexpr (KIND == K_SIDDON_MR)
@@ -566,6 +576,18 @@ struct Fixed
 	const unsigned* maxBits;  // M as float bits (pass 1 result)
 	uint64_t n;               // events (bins) of the call
 };
+
+// Siddon rays: |w| is a segment's length (times at most the TOF peak), and a
+// segment lies between two planes of each axis one voxel apart, so it is not
+// longer than the voxel's diagonal; a first plane misplaced by one in FP32
+// doubles that.  Twice as much again as margin: M may be too large (2 bits of
+// the 61 per factor of 4), not too small.  Knowing it, the bound of a value
+// given per event needs no walk.
+__host__ __device__ inline float siddonWeightBound(const KParams& P, bool tof)
+{
+	const float d = sqrtf(P.g.vx * P.g.vx + P.g.vy * P.g.vy + P.g.vz * P.g.vz);
+	return 4.f * d * (tof ? P.tof.norm : 1.f);
+}
 
 // Exponent k with n * M < 2^k; 0x7fffffff when M is zero or not finite.
 __device__ __forceinline__ int fixedExponent(unsigned maxBits, uint64_t n)
@@ -620,7 +642,7 @@ __device__ __forceinline__ void redV2(float* p, float2 v)
 // The last group of an image whose size is no multiple of 4 (or the last pair
 // of an odd one) is sent voxel by voxel: whole groups are those below `whole`.
 template <int KIND, bool TOF, bool COMP, bool FIX = false, int VEC = 0,
-          bool TILE = false>
+          bool TILE = false, bool WARP = false>
 __device__ __forceinline__ void backwardEvent(const KParams& P,
                                               float* __restrict__ img,
                                               float v, float3 p1, float3 p2,
@@ -630,7 +652,7 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
                                               double scale = 0.0, int part = 0,
                                               int parts = 1,
                                               float* vslot = nullptr,
-                                              int vstride = 0)
+                                              int vstride = 0, bool alive = true)
 {
 	if constexpr (KIND == K_SIDDON_MR)
 		v = v / static_cast<float>(P.numRays);
@@ -643,8 +665,15 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
 			const long long q = __double2ll_rn(vs * static_cast<double>(w));
 			atomicAdd(fix + o, static_cast<unsigned long long>(q));
 		};
-		projectEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2, tofv, rid, false, visit,
-		                              endRay, part, parts);
+		projectEvent<KIND, TOF, COMP, false, WARP>(P, p1, p2, n1, n2, tofv, rid, false,
+		                                           visit, endRay, part, parts, alive);
+	}
+	else if constexpr (KIND == K_DD_PSF && COMP && VEC != 0)
+	{
+		auto quad = [&](int o, float4 w)
+		{ redV4(img + o, make_float4(v * w.x, v * w.y, v * w.z, v * w.w)); };
+		projectEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2, tofv, rid, false, quad, endRay, part,
+		                              parts);
 	}
 	else if constexpr (VEC == 2)
 	{
@@ -772,8 +801,8 @@ __device__ __forceinline__ void backwardEvent(const KParams& P,
 	else
 	{
 		auto visit = [&](int o, float w) { atomicAdd(img + o, v * w); };
-		projectEvent<KIND, TOF, COMP, TILE>(P, p1, p2, n1, n2, tofv, rid, false, visit,
-		                                    endRay, part, parts);
+		projectEvent<KIND, TOF, COMP, TILE, WARP>(P, p1, p2, n1, n2, tofv, rid, false, visit,
+		                                          endRay, part, parts, alive);
 	}
 }
 
@@ -1028,7 +1057,9 @@ __global__ void __launch_bounds__(kBlock, KIND == K_SIDDON ? 4 : 1)
 			if constexpr (!EM)
 			{
 				const float v = __ldg(in + e);
-				if (v != 0.f)
+				if constexpr (KIND == K_SIDDON || KIND == K_SIDDON_MR)
+					b = fabsf(v) * siddonWeightBound(P, TOF);
+				else if (v != 0.f)
 					b = fabsf(v) * maxWeightEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2,
 					                                                tofv, k);
 			}
@@ -1339,119 +1370,299 @@ __global__ void __launch_bounds__(kBlock)
 	}
 }
 
-// Histogram-bin kernels: sensitivity back projection and histogram EM.
-// MODE H_BOUND is pass 1 and H_FIX pass 2 of the deterministic back
-// projection (see Fixed); H_PLAIN scatters floats.
+// Histogram-bin kernels: sensitivity back projection, histogram EM, and the
+// forward and back projection of values given per bin.  MODE H_BOUND is pass
+// 1 and H_FIX pass 2 of the deterministic back projection (see Fixed); H_PLAIN
+// scatters floats.
 enum HistoMode
 {
 	H_PLAIN = 0,
 	H_BOUND = 1,
 	H_FIX = 2
 };
+enum HistoOp
+{
+	HOP_SENS = 0,  // out += A^T (sens * acf)
+	HOP_EM = 1,    // out += A^T (meas / model)
+	HOP_FWD = 2,   // vals[bin] = A img
+	HOP_BWD = 3    // out += A^T vals[bin]
+};
+
+struct HistoArgs
+{
+	uint64_t count, numPhiSubset, numSubsets, subset;
+	const float* img;
+	float* out;
+	const float* meas;
+	const float* sensH;
+	const float* acfH;
+	const float* addH;
+	Geom mu;
+	const float* muImg;
+	float globalScale, denomThr;
+	Fixed F;
+	unsigned* maxBits;
+	const uint64_t* list;
+	const float* crystalEff;
+	float* vals;
+	// HOP_SENS in two passes: the bins' values, written by pass 1 (with their
+	// walk through the attenuation image) and read by pass 2; or null.
+	float* stored;
+};
 
 // Blocks per SM of the compensated DD + PSF histogram EM kernel (several
 // threads per bin).
 constexpr int kDDPsfBlocksPerSM = 2;
-template <int KIND, bool EM, int MODE = H_PLAIN, bool COMP = false, int TPL = 1>
-__global__ void __launch_bounds__(kBlock, (KIND == K_DD_PSF && TPL > 1) ? kDDPsfBlocksPerSM : 1)
-    k_histo(KParams P, H3Dev H, uint64_t count, uint64_t numPhiSubset,
-            uint64_t numSubsets, uint64_t subset, const float* __restrict__ img,
-            float* __restrict__ out, const float* __restrict__ meas,
-            const float* __restrict__ sensH, const float* __restrict__ acfH,
-            const float* __restrict__ addH, Geom mu,
-            const float* __restrict__ muImg, float globalScale, float denomThr,
-            Fixed F, unsigned* maxBits, const uint64_t* __restrict__ list,
-            const float* __restrict__ crystalEff)
+
+// Item t (ok: it exists) of a histogram operation: subset-local bin t, or
+// list[t] with a list (which then holds only the bins that do work).
+// TPL > 1: lane j of a group walks piece j of the bin's rows; the forward
+// partial sums are added over the group, which then shares the EM ratio.
+// Siddon rays (the image's and the attenuation image's) are walked in lock
+// step, so every lane of a warp calls this: the bins of a warp are neighbours
+// in r, whose rays run side by side but step along different axes at
+// different times, and walked freely they drift apart.
+template <int KIND, int HOP, int MODE, bool COMP, int TPL>
+__device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, const HistoArgs& A,
+                                          uint64_t t, bool ok, int part)
 {
-	static_assert(TPL == 1 || (KIND == K_DD_PSF && EM && MODE == H_PLAIN && COMP),
+	static_assert(TPL == 1 || (KIND == K_DD_PSF && HOP == HOP_EM && MODE == H_PLAIN && COMP),
 	              "several threads per bin: compensated DD + PSF histogram EM");
-	// One item per TPL threads: a warp's threads stay converged across items
-	// (a grid-stride loop lets them drift apart between items).  With a list,
-	// item t is the subset-local bin index list[t] (count = list length), so
-	// that warps hold only the bins that do work.  TPL > 1: lane j of a group
-	// walks piece j of the bin's rows; the forward partial sums are added over
-	// the group, which then shares the EM ratio.
-	const uint64_t gt = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-	const uint64_t t = gt / TPL;
-	const int part = static_cast<int>(gt % TPL);
-	float bound = 0.f;  // H_BOUND: |v| * max|w| of this bin
-	do
+	static_assert(HOP != HOP_FWD || MODE == H_PLAIN, "forward projection scatters nothing");
+	constexpr bool WARP = KIND == K_SIDDON;
+	constexpr bool EM = HOP == HOP_EM;
+	const bool exists = ok;
+	uint64_t k = 0, bin = 0;
+	uint32_t d1 = 0, d2 = 0;
+	if (ok)
 	{
-		if (t >= count)
-			break;
-		const uint64_t k = list ? __ldg(list + t) : t;
-		const uint64_t bin = h3SubsetBin(H, k, numPhiSubset, numSubsets, subset);
-		uint32_t d1, d2;
+		k = A.list ? __ldg(A.list + t) : t;
+		bin = h3SubsetBin(H, k, A.numPhiSubset, A.numSubsets, A.subset);
 		h3Pair(H, bin, d1, d2);
-		if (d1 == 0 && d2 == 0)
-			break;
-		const float m = EM ? __ldg(meas + bin) : 1.0f;
-		if (EM && m == 0.f)
-			break;
-		// LOR sensitivity: a histogram value, or the product of the two
-		// crystals' factors (the same FP32 product a histogram of them holds).
-		const float s = sensH ? __ldg(sensH + bin) :
-		                (crystalEff ? __ldg(crystalEff + d1) * __ldg(crystalEff + d2) : 1.0f);
+		ok = !(d1 == 0 && d2 == 0);
+		if (HOP == HOP_FWD && !ok)
+			A.vals[bin] = 0.f;
+	}
+	const float m = (EM && ok) ? __ldg(A.meas + bin) : 1.0f;
+	ok = ok && !(EM && m == 0.f);
+	float3 p1 = make_float3(0.f, 0.f, 0.f), p2 = p1, n1 = p1, n2 = p1;
+	if (ok)
+	{
 		const float4 pa = __ldg(P.scan.pos + d1), pb = __ldg(P.scan.pos + d2);
-		const float4 oa = __ldg(P.scan.ori + d1), ob = __ldg(P.scan.ori + d2);
-		float3 p1 = make_float3(pa.x, pa.y, pa.z), p2 = make_float3(pb.x, pb.y, pb.z);
-		const float3 n1 = make_float3(oa.x, oa.y, oa.z), n2 = make_float3(ob.x, ob.y, ob.z);
-		float a = 1.0f;
-		if (acfH)
+		p1 = make_float3(pa.x, pa.y, pa.z);
+		p2 = make_float3(pb.x, pb.y, pb.z);
+		if constexpr (KIND != K_SIDDON)
 		{
-			a = __ldg(acfH + bin);
+			const float4 oa = __ldg(P.scan.ori + d1), ob = __ldg(P.scan.ori + d2);
+			n1 = make_float3(oa.x, oa.y, oa.z);
+			n2 = make_float3(ob.x, ob.y, ob.z);
 		}
-		else if (muImg)
+	}
+	// LOR sensitivity: a histogram value, or the product of the two crystals'
+	// factors (the same FP32 product a histogram of them holds).
+	float s = 1.f, a = 1.f, v = 0.f;
+	const bool ready = HOP == HOP_SENS && MODE == H_FIX && A.stored != nullptr;
+	if (HOP == HOP_BWD)
+	{
+		v = ok ? __ldg(A.vals + bin) : 0.f;
+	}
+	else if (ready)
+	{
+		v = ok ? __ldg(A.stored + t) : 0.f;
+	}
+	else if (HOP != HOP_FWD)
+	{
+		if (ok)
+			s = A.sensH ? __ldg(A.sensH + bin)
+			            : (A.crystalEff ? __ldg(A.crystalEff + d1) * __ldg(A.crystalEff + d2)
+			                            : 1.0f);
+		if (A.acfH)
 		{
+			a = ok ? __ldg(A.acfH + bin) : 1.f;
+		}
+		else if (A.muImg)  // uniform over the launch
+		{
+			// The image reads of 8 crossings in flight together, summed in
+			// walk order (as the attenuation factors of events).
 			float acc = 0.f;
-			auto visit = [&](int o, float w) { acc += w * __ldg(muImg + o); };
-			const float3 mo = make_float3(mu.offx, mu.offy, mu.offz);
-			siddonWalk<false, false>(mu, f3sub(p1, mo), f3sub(p2, mo), P.tof, 0.f, visit);
+			constexpr int B = attBatch<false>();
+			auto consume = [&](const int (&o)[B], const float (&w)[B])
+			{
+				float q[B];
+#pragma unroll
+				for (int j = 0; j < B; j++)
+					q[j] = o[j] >= 0 ? __ldg(A.muImg + o[j]) : 0.f;
+#pragma unroll
+				for (int j = 0; j < B; j++)
+					if (o[j] >= 0)
+						acc += w[j] * q[j];
+			};
+			const float3 mo = make_float3(A.mu.offx, A.mu.offy, A.mu.offz);
+			siddonWalkWarpBatched<false, false, B>(ok, A.mu, f3sub(p1, mo), f3sub(p2, mo), P.tof,
+			                                       0.f, consume);
 			a = expf(-acc * 0.1f);
 		}
-		const float3 off = make_float3(P.g.offx, P.g.offy, P.g.offz);
-		p1 = f3sub(p1, off);
-		p2 = f3sub(p2, off);
-		float v = a * s;
-		float mw = 0.f;
-		if constexpr (EM)
+		v = a * s;
+	}
+	const float3 off = make_float3(P.g.offx, P.g.offy, P.g.offz);
+	p1 = f3sub(p1, off);
+	p2 = f3sub(p2, off);
+	float bound = 0.f;  // H_BOUND: |v| * max|w| of this bin
+	if constexpr (EM || HOP == HOP_FWD)
+	{
+		float mw = 0.f, u = 0.f;
+		if (WARP || ok)
+			u = forwardEvent<KIND, false, COMP, MODE == H_BOUND, false, false, WARP>(
+			    P, A.img, p1, p2, n1, n2, 0.f, k, MODE == H_BOUND ? &mw : nullptr, part, TPL, ok);
+		if constexpr (TPL > 1)
+			if (ok)  // the lanes of a group share the bin
+				u = groupSum<TPL>(u);
+		if constexpr (HOP == HOP_FWD)
 		{
-			float u;
-			if constexpr (MODE == H_BOUND)
-				u = forwardEvent<KIND, false, COMP, true>(P, img, p1, p2, n1, n2,
-				                                          0.f, k, &mw);
-			else
-				u = groupSum<TPL>(forwardEvent<KIND, false, COMP>(
-				    P, img, p1, p2, n1, n2, 0.f, k, nullptr, part, TPL));
-			u *= s;
-			u *= a;
-			u *= globalScale;
-			if (addH)
-				u += __ldg(addH + bin);
-			if (!(fabsf(u) > denomThr))
-				break;
-			u = m / u;
-			u *= s;
-			u *= a;
-			u *= globalScale;
-			v = u;
+			if (ok)
+				A.vals[bin] = u;
+			return;
 		}
-		else if constexpr (MODE == H_BOUND)
-		{
-			if (v != 0.f)
-				mw = maxWeightEvent<KIND, false, COMP>(P, p1, p2, n1, n2, 0.f, k);
-		}
+		u *= s;
+		u *= a;
+		u *= A.globalScale;
+		if (A.addH && ok)
+			u += __ldg(A.addH + bin);
+		ok = ok && fabsf(u) > A.denomThr;
+		u = m / u;
+		u *= s;
+		u *= a;
+		u *= A.globalScale;
+		v = u;
 		if constexpr (MODE == H_BOUND)
-			bound = fabsf(v) * mw;
-		else if constexpr (MODE == H_FIX)
-			backwardEvent<KIND, false, COMP, true>(P, nullptr, v, p1, p2, n1, n2,
-			                                       0.f, k, F.acc, fixedScale(F));
-		else
-			backwardEvent<KIND, false, COMP>(P, out, v, p1, p2, n1, n2, 0.f, k, nullptr,
-			                                 0.0, part, TPL);
-	} while (false);
+			bound = ok ? fabsf(v) * mw : 0.f;
+	}
+	else if constexpr (MODE == H_BOUND)
+	{
+		if (A.stored && exists)
+			A.stored[t] = v;
+		if (ok)
+		{
+			if constexpr (KIND == K_SIDDON || KIND == K_SIDDON_MR)
+				bound = fabsf(v) * siddonWeightBound(P, false);
+			else
+				bound = fabsf(v) *
+				        (v != 0.f ? maxWeightEvent<KIND, false, COMP>(P, p1, p2, n1, n2, 0.f, k)
+				                  : 0.f);
+		}
+	}
 	if constexpr (MODE == H_BOUND)
-		warpMaxInto(maxBits, bound != bound ? __uint_as_float(0x7fffffffu) : bound);
+	{
+		warpMaxInto(A.maxBits, bound != bound ? __uint_as_float(0x7fffffffu) : bound);
+	}
+	else if constexpr (MODE == H_FIX)
+	{
+		if (WARP || ok)
+			backwardEvent<KIND, false, COMP, true, 0, false, WARP>(
+			    P, nullptr, v, p1, p2, n1, n2, 0.f, k, A.F.acc, fixedScale(A.F), 0, 1, nullptr, 0,
+			    ok);
+	}
+	else
+	{
+		if (WARP || ok)
+			backwardEvent<KIND, false, COMP, false, 0, false, WARP>(
+			    P, A.out, v, p1, p2, n1, n2, 0.f, k, nullptr, 0.0, part, TPL, nullptr, 0, ok);
+	}
+}
+
+// One item per TPL threads: a warp's threads stay converged across items (a
+// grid-stride loop lets them drift apart between items).
+template <int KIND, int HOP, int MODE = H_PLAIN, bool COMP = false, int TPL = 1>
+__global__ void __launch_bounds__(kBlock, (KIND == K_DD_PSF && TPL > 1) ? kDDPsfBlocksPerSM : 1)
+    k_histo(KParams P, H3Dev H, const __grid_constant__ HistoArgs A)
+{
+	const uint64_t gt = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+	histoItem<KIND, HOP, MODE, COMP, TPL>(P, H, A, gt / TPL, gt / TPL < A.count,
+	                                             static_cast<int>(gt % TPL));
+}
+
+// Single-ray Siddon: a block takes kSiddonTile items, lists those whose ray
+// crosses the grid, in order, and walks the list.  On 256 x 16 crystals of 300
+// mm radius and a 256 mm field only 27 % of the bins cross it, in runs of 35
+// of 127 neighbours, so that one bin per thread left 13 of 32 lanes of the
+// working warps without a ray.  384 items give 128 threads about one list's
+// worth there and about two where most bins cross.  693,000 bins, 128 x 128 x
+// 64 voxels, lock step without and with the list: forward 258 -> 127 us, back
+// 209 -> 175 us; the attenuated sensitivity image's first pass 1.99 -> 1.15 ms,
+// its second 1.74 -> 1.95 (64-bit reductions at the L2's limit).
+constexpr int kSiddonBlock = 128, kSiddonTile = 3 * kSiddonBlock;
+template <int HOP, int MODE, bool COMP>
+__global__ void __launch_bounds__(kSiddonBlock, 8)
+    k_histo_siddon(KParams P, H3Dev H, const __grid_constant__ HistoArgs A)
+{
+	__shared__ uint16_t list[kSiddonTile];
+	__shared__ int warpCount[kSiddonBlock / 32];
+	const uint64_t first = static_cast<uint64_t>(blockIdx.x) * kSiddonTile;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	int n = 0;
+	float idle = 0.f;  // H_BOUND: NaN if a bin without a walk has no finite value
+#pragma unroll
+	for (int i = 0; i < kSiddonTile; i += kSiddonBlock)
+	{
+		const uint64_t t = first + i + threadIdx.x;
+		bool in = false;
+		if (t < A.count)
+		{
+			const uint64_t k = A.list ? __ldg(A.list + t) : t;
+			const uint64_t bin = h3SubsetBin(H, k, A.numPhiSubset, A.numSubsets, A.subset);
+			uint32_t d1, d2;
+			h3Pair(H, bin, d1, d2);
+			const bool pair = !(d1 == 0 && d2 == 0);
+			if (pair)
+			{
+				const float4 pa = __ldg(P.scan.pos + d1), pb = __ldg(P.scan.pos + d2);
+				const float3 off = make_float3(P.g.offx, P.g.offy, P.g.offz);
+				in = crossesGrid(P.g, f3sub(make_float3(pa.x, pa.y, pa.z), off),
+				                 f3sub(make_float3(pb.x, pb.y, pb.z), off));
+			}
+			if (HOP == HOP_FWD && !in)
+				A.vals[bin] = 0.f;
+			if (MODE == H_BOUND && pair && !in)
+			{
+				if (HOP == HOP_BWD)
+					idle += 0.f * __ldg(A.vals + bin);
+				if (HOP == HOP_SENS && A.sensH)
+					idle += 0.f * __ldg(A.sensH + bin);
+				if (HOP == HOP_SENS && A.acfH)
+					idle += 0.f * __ldg(A.acfH + bin);
+				if (HOP == HOP_EM && A.addH)
+				{
+					// The ratio of a bin whose model is its additive term.
+					const float m = __ldg(A.meas + bin), u = __ldg(A.addH + bin);
+					const float c = (A.sensH ? __ldg(A.sensH + bin) : 1.f) *
+					                (A.acfH ? __ldg(A.acfH + bin) : 1.f) * A.globalScale;
+					if (m != 0.f && fabsf(u) > A.denomThr)
+						idle += 0.f * (m / u * c);
+				}
+			}
+		}
+		const unsigned ballot = __ballot_sync(0xffffffffu, in);
+		if (lane == 0)
+			warpCount[warp] = __popc(ballot);
+		__syncthreads();
+		int at = n + __popc(ballot & ((1u << lane) - 1u));
+		for (int w = 0; w < kSiddonBlock / 32; w++)
+		{
+			if (w < warp)
+				at += warpCount[w];
+			n += warpCount[w];
+		}
+		if (in)
+			list[at] = static_cast<uint16_t>(i + threadIdx.x);
+		__syncthreads();
+	}
+	if (MODE == H_BOUND && idle != idle)
+		atomicMax(A.maxBits, 0x7fffffffu);
+	for (int j = warp * 32; j < n; j += kSiddonBlock)  // uniform over a warp
+	{
+		const bool ok = j + lane < n;
+		histoItem<K_SIDDON, HOP, MODE, COMP, 1>(P, H, A, first + (ok ? list[j + lane] : 0), ok, 0);
+	}
 }
 
 // 8-bit value spread to every third bit (Morton interleave).
@@ -3042,90 +3253,132 @@ struct NonzeroBin
 	}
 };
 
-template <bool EM>
-yrtb_status dispatchHisto(yrtb_projector* h, int numSubsets, int subset,
-                          const float* img, float* out, const float* meas,
-                          const float* sensH, const float* acfH,
-                          const float* addH, const float* mu,
-                          const yrtb_image_params* muParams, float gs,
-                          float thr, yrtb_stream stream,
-                          const uint64_t* list = nullptr, uint64_t listCount = 0,
-                          const float* crystalEff = nullptr)
+// Largest array of bin values kept between the two passes of a deterministic
+// sensitivity image; larger subsets walk the attenuation image in both.
+constexpr uint64_t kStoredBytes = uint64_t(512) << 20;
+
+// Runs one histogram operation over a subset's bins, or the listed ones.  A
+// holds the operation's buffers; the subset and the two-pass fields are set
+// here.
+template <int HOP>
+yrtb_status dispatchHisto(yrtb_projector* h, int numSubsets, int subset, HistoArgs A,
+                          const yrtb_image_params* muParams, yrtb_stream stream,
+                          uint64_t listCount = 0)
 {
-	if (!h || !out || numSubsets <= 0 || subset < 0 || subset >= numSubsets)
+	constexpr bool kScatter = HOP != HOP_FWD;
+	if (!h || (kScatter && !A.out) || numSubsets <= 0 || subset < 0 || subset >= numSubsets)
 		return fail(YRTB_ERR_ARGUMENT, "invalid histogram subset or buffers");
-	if (EM && (!img || !meas))
+	if (HOP == HOP_EM && (!A.img || !A.meas))
 		return fail(YRTB_ERR_ARGUMENT, "histogram EM needs image and measurements");
-	if (mu && !validImage(muParams))
+	if (A.muImg && !validImage(muParams))
 		return fail(YRTB_ERR_ARGUMENT, "attenuation image needs valid parameters");
-	if (h->ip.nt != 1)
+	// The operators read and add to the first frame, as list-mode projection
+	// of events without frames does.
+	if ((HOP == HOP_SENS || HOP == HOP_EM) && h->ip.nt != 1)
 		return fail(YRTB_ERR_ARGUMENT, "histogram-mode projection is single-frame");
 	YRTB_CUDA(cudaSetDevice(h->device));
-	uint64_t nps = 0;
-	const uint64_t subsetCount = h3SubsetSize(*h->h3, numSubsets, subset, nps);
+	A.numSubsets = static_cast<uint64_t>(numSubsets);
+	A.subset = static_cast<uint64_t>(subset);
+	const uint64_t subsetCount = h3SubsetSize(*h->h3, A.numSubsets, A.subset, A.numPhiSubset);
 	// Threads: one per listed bin, or one per bin of the subset.  The
 	// fixed-point scale of deterministic mode is set by the subset size in
 	// both forms, so that they give the same image.
-	const uint64_t count = list ? listCount : subsetCount;
-	const Geom mg = mu ? makeGeom(*muParams) : Geom{};
+	A.count = A.list ? listCount : subsetCount;
+	A.mu = A.muImg ? makeGeom(*muParams) : Geom{};
+	A.maxBits = h->d_fixMax;
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-	const unsigned grid = gridAll(count);
-	Fixed F{};
-	if (h->det)
+	if (A.count == 0)
+		return YRTB_OK;
+	const unsigned grid = gridAll(A.count);
+	const bool det = kScatter && h->det;
+	if (det)
 	{
-		const yrtb_status s = fixedBegin(h, subsetCount, st, F);
+		const yrtb_status s = fixedBegin(h, subsetCount, st, A.F);
 		if (s != YRTB_OK)
 			return s;
+		// Pass 1 keeps the values whose attenuation it walked for pass 2; with
+		// no room for them, pass 2 walks again.
+		if (HOP == HOP_SENS && A.muImg && !A.acfH && A.count * sizeof(float) <= kStoredBytes &&
+		    poolAlloc(&A.stored, A.count * sizeof(float), st) != cudaSuccess)
+		{
+			A.stored = nullptr;
+			(void)cudaGetLastError();
+		}
 	}
 	auto launch = [&](auto kind, auto comp)
 	{
 		constexpr int K = decltype(kind)::value;
 		constexpr bool C = decltype(comp)::value;
-		if (h->det)
+		if constexpr (K == K_SIDDON)
 		{
-			k_histo<K, EM, H_BOUND, C><<<grid, kBlock, 0, st>>>(
-			    h->P, h->h3d, count, nps, numSubsets, subset, img, out, meas, sensH,
-			    acfH, addH, mg, mu, gs, thr, F, h->d_fixMax, list, crystalEff);
-			k_histo<K, EM, H_FIX, C><<<grid, kBlock, 0, st>>>(
-			    h->P, h->h3d, count, nps, numSubsets, subset, img, out, meas, sensH,
-			    acfH, addH, mg, mu, gs, thr, F, nullptr, list, crystalEff);
+			const unsigned tiles =
+			    static_cast<unsigned>((A.count + kSiddonTile - 1) / kSiddonTile);
+			if constexpr (kScatter)
+			{
+				if (h->det)
+				{
+					k_histo_siddon<HOP, H_BOUND, C><<<tiles, kSiddonBlock, 0, st>>>(h->P, h->h3d,
+					                                                               A);
+					k_histo_siddon<HOP, H_FIX, C><<<tiles, kSiddonBlock, 0, st>>>(h->P, h->h3d, A);
+					return;
+				}
+			}
+			k_histo_siddon<HOP, H_PLAIN, C><<<tiles, kSiddonBlock, 0, st>>>(h->P, h->h3d, A);
+			return;
 		}
-		else if constexpr (EM && K == K_DD_PSF && C)
+		if constexpr (kScatter && K != K_SIDDON)
+		{
+			if (h->det)
+			{
+				k_histo<K, HOP, H_BOUND, C><<<grid, kBlock, 0, st>>>(h->P, h->h3d, A);
+				k_histo<K, HOP, H_FIX, C><<<grid, kBlock, 0, st>>>(h->P, h->h3d, A);
+				return;
+			}
+		}
+		if constexpr (K == K_SIDDON)
+		{
+		}
+		else if constexpr (HOP == HOP_EM && K == K_DD_PSF && C)
 		{
 			// Compensated DD + PSF EM: kHistoDDThreads threads per bin, each
 			// on an even share of the bin's rows.
 			constexpr int T = kHistoDDThreads;
-			k_histo<K, EM, H_PLAIN, C, T><<<gridAll(count * T), kBlock, 0, st>>>(
-			    h->P, h->h3d, count, nps, numSubsets, subset, img, out, meas, sensH,
-			    acfH, addH, mg, mu, gs, thr, F, nullptr, list, crystalEff);
+			k_histo<K, HOP, H_PLAIN, C, T><<<gridAll(A.count * T), kBlock, 0, st>>>(h->P, h->h3d,
+			                                                                       A);
 		}
 		else
 		{
-			k_histo<K, EM, H_PLAIN, C><<<grid, kBlock, 0, st>>>(
-			    h->P, h->h3d, count, nps, numSubsets, subset, img, out, meas, sensH,
-			    acfH, addH, mg, mu, gs, thr, F, nullptr, list, crystalEff);
+			k_histo<K, HOP, H_PLAIN, C><<<grid, kBlock, 0, st>>>(h->P, h->h3d, A);
 		}
 	};
-	// Histogram mode honours the precision for single-ray Siddon and DD + PSF.
+	// Sensitivity and EM honour the precision for single-ray Siddon and DD +
+	// PSF; the operators also for multi-ray, as on events.
+	constexpr bool kOperator = HOP == HOP_FWD || HOP == HOP_BWD;
+	auto either = [&](auto kind)
+	{
+		if (h->comp)
+			launch(kind, std::true_type{});
+		else
+			launch(kind, std::false_type{});
+	};
 	switch (h->kind)
 	{
-	case K_SIDDON:
-		if (h->comp)
-			launch(std::integral_constant<int, K_SIDDON>{}, std::true_type{});
+	case K_SIDDON: either(std::integral_constant<int, K_SIDDON>{}); break;
+	case K_SIDDON_MR:
+		if constexpr (kOperator)
+			either(std::integral_constant<int, K_SIDDON_MR>{});
 		else
-			launch(std::integral_constant<int, K_SIDDON>{}, std::false_type{});
+			launch(std::integral_constant<int, K_SIDDON_MR>{}, std::false_type{});
 		break;
-	case K_SIDDON_MR: launch(std::integral_constant<int, K_SIDDON_MR>{}, std::false_type{}); break;
 	case K_DD: launch(std::integral_constant<int, K_DD>{}, std::false_type{}); break;
-	default:
-		if (h->comp)
-			launch(std::integral_constant<int, K_DD_PSF>{}, std::true_type{});
-		else
-			launch(std::integral_constant<int, K_DD_PSF>{}, std::false_type{});
-		break;
+	default: either(std::integral_constant<int, K_DD_PSF>{}); break;
 	}
-	if (h->det)
-		fixedEnd(h, F, out, st);
+	if (det)
+	{
+		if (A.stored)
+			cudaFreeAsync(A.stored, st);
+		fixedEnd(h, A.F, A.out, st);
+	}
 	YRTB_LAUNCHED();
 	return YRTB_OK;
 }
@@ -4113,9 +4366,12 @@ yrtb_status yrtb_sensitivity_histo3d(yrtb_projector* h, float* d_sens,
 {
 	if (!h || !h->h3)
 		return fail(YRTB_ERR_ARGUMENT, "projector has no Histogram3D (odd ring)");
-	return dispatchHisto<false>(h, num_subsets, subset, nullptr, d_sens, nullptr,
-	                            d_sens_histo, d_acf_histo, nullptr, d_mu,
-	                            mu_params, 1.f, 0.f, stream);
+	HistoArgs A{};
+	A.out = d_sens;
+	A.sensH = d_sens_histo;
+	A.acfH = d_acf_histo;
+	A.muImg = d_mu;
+	return dispatchHisto<HOP_SENS>(h, num_subsets, subset, A, mu_params, stream);
 }
 
 yrtb_status yrtb_sensitivity_histo3d_crystal(yrtb_projector* h, float* d_sens,
@@ -4130,9 +4386,12 @@ yrtb_status yrtb_sensitivity_histo3d_crystal(yrtb_projector* h, float* d_sens,
 		return fail(YRTB_ERR_ARGUMENT, "projector has no Histogram3D (odd ring)");
 	if (!d_crystal_eff)
 		return fail(YRTB_ERR_ARGUMENT, "null crystal factors");
-	return dispatchHisto<false>(h, num_subsets, subset, nullptr, d_sens, nullptr,
-	                            nullptr, d_acf_histo, nullptr, d_mu, mu_params,
-	                            1.f, 0.f, stream, nullptr, 0, d_crystal_eff);
+	HistoArgs A{};
+	A.out = d_sens;
+	A.crystalEff = d_crystal_eff;
+	A.acfH = d_acf_histo;
+	A.muImg = d_mu;
+	return dispatchHisto<HOP_SENS>(h, num_subsets, subset, A, mu_params, stream);
 }
 
 yrtb_status yrtb_gather_crystal_product(yrtb_projector* h,
@@ -4158,6 +4417,59 @@ yrtb_status yrtb_gather_crystal_product(yrtb_projector* h,
 	return YRTB_OK;
 }
 
+// The arguments the operators on histogram bins share.
+static yrtb_status histoOperator(yrtb_projector* h, const void* image, const void* values)
+{
+	if (!h || !h->h3)
+		return fail(YRTB_ERR_ARGUMENT, "projector has no Histogram3D (odd ring)");
+	if (!image || !values)
+		return fail(YRTB_ERR_ARGUMENT, "null image or values");
+	if (h->hasTof)
+		return fail(YRTB_ERR_ARGUMENT, "TOF projector requires per-event TOF values");
+	if (h->layout != YRTB_LAYOUT_ROW_MAJOR)
+		return fail(YRTB_ERR_ARGUMENT, "histogram projection takes row-major images");
+	return YRTB_OK;
+}
+
+yrtb_status yrtb_forward_histo3d(yrtb_projector* h, const float* d_image, int num_subsets,
+                                 int subset, float* d_values, yrtb_stream stream)
+{
+	const yrtb_status s = histoOperator(h, d_image, d_values);
+	if (s != YRTB_OK)
+		return s;
+	HistoArgs A{};
+	A.img = d_image;
+	A.vals = d_values;
+	return dispatchHisto<HOP_FWD>(h, num_subsets, subset, A, nullptr, stream);
+}
+
+yrtb_status yrtb_backward_histo3d(yrtb_projector* h, const float* d_values, int num_subsets,
+                                  int subset, float* d_image, yrtb_stream stream)
+{
+	const yrtb_status s = histoOperator(h, d_image, d_values);
+	if (s != YRTB_OK)
+		return s;
+	HistoArgs A{};
+	A.out = d_image;
+	A.vals = const_cast<float*>(d_values);  // read only
+	return dispatchHisto<HOP_BWD>(h, num_subsets, subset, A, nullptr, stream);
+}
+
+static HistoArgs emArgs(const float* image, float* em, const float* meas, const float* sens,
+                        const float* acf, const float* add, float gs, float thr)
+{
+	HistoArgs A{};
+	A.img = image;
+	A.out = em;
+	A.meas = meas;
+	A.sensH = sens;
+	A.acfH = acf;
+	A.addH = add;
+	A.globalScale = gs;
+	A.denomThr = thr;
+	return A;
+}
+
 yrtb_status yrtb_em_step_histo3d(yrtb_projector* h, const float* d_image,
                                  float* d_em, const float* d_meas,
                                  const float* d_sens_histo,
@@ -4168,9 +4480,10 @@ yrtb_status yrtb_em_step_histo3d(yrtb_projector* h, const float* d_image,
 {
 	if (!h || !h->h3)
 		return fail(YRTB_ERR_ARGUMENT, "projector has no Histogram3D (odd ring)");
-	return dispatchHisto<true>(h, num_subsets, subset, d_image, d_em, d_meas,
-	                           d_sens_histo, d_acf_histo, d_add_histo, nullptr,
-	                           nullptr, global_scale, denom_threshold, stream);
+	return dispatchHisto<HOP_EM>(h, num_subsets, subset,
+	                             emArgs(d_image, d_em, d_meas, d_sens_histo, d_acf_histo,
+	                                    d_add_histo, global_scale, denom_threshold),
+	                             nullptr, stream);
 }
 
 yrtb_status yrtb_histo3d_subset_nonzero(yrtb_projector* h, const float* d_meas,
@@ -4239,9 +4552,10 @@ yrtb_status yrtb_em_step_histo3d_list(yrtb_projector* h, const float* d_image,
 		return fail(YRTB_ERR_ARGUMENT, "null bin list");
 	if (n == 0)
 		return YRTB_OK;
-	return dispatchHisto<true>(h, num_subsets, subset, d_image, d_em, d_meas,
-	                           d_sens_histo, d_acf_histo, d_add_histo, nullptr,
-	                           nullptr, global_scale, denom_threshold, stream, d_k, n);
+	HistoArgs A = emArgs(d_image, d_em, d_meas, d_sens_histo, d_acf_histo, d_add_histo,
+	                     global_scale, denom_threshold);
+	A.list = d_k;
+	return dispatchHisto<HOP_EM>(h, num_subsets, subset, A, nullptr, stream, n);
 }
 
 yrtb_status yrtb_listmode_to_histo3d(yrtb_projector* h, const uint32_t* d1,

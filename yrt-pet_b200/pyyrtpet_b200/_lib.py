@@ -148,6 +148,10 @@ SIGNATURES = {
                                           ctypes.c_int, c_vp], ctypes.c_int),
     "yrtb_gather_crystal_product": ([c_vp, c_vp, _P(yrtb_events), yrtb_range,
                                      c_vp, c_vp], ctypes.c_int),
+    "yrtb_forward_histo3d": ([c_vp, c_vp, ctypes.c_int, ctypes.c_int, c_vp, c_vp],
+                             ctypes.c_int),
+    "yrtb_backward_histo3d": ([c_vp, c_vp, ctypes.c_int, ctypes.c_int, c_vp, c_vp],
+                              ctypes.c_int),
     "yrtb_em_step_histo3d": ([c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp,
                               ctypes.c_int, ctypes.c_int, c_f, c_f, c_vp],
                              ctypes.c_int),

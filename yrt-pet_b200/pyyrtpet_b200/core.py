@@ -934,6 +934,20 @@ class DeviceProjector:
             _ptr(mu), mp, int(num_subsets), int(subset), _stream()))
         return sens_img
 
+    def forward_histo3d(self, img, values, num_subsets=1, subset=0):
+        """values[bin] = A img over one subset of the histogram's bins."""
+        self._check_image(img)
+        L.check(L.lib().yrtb_forward_histo3d(self.h, img.data_ptr(), int(num_subsets),
+                                             int(subset), values.data_ptr(), _stream()))
+        return values
+
+    def backward_histo3d(self, values, img, num_subsets=1, subset=0):
+        """img += A^T values over one subset of the histogram's bins."""
+        self._check_image(img)
+        L.check(L.lib().yrtb_backward_histo3d(self.h, values.data_ptr(), int(num_subsets),
+                                              int(subset), img.data_ptr(), _stream()))
+        return img
+
     def em_step_histo3d(self, img, em, meas, num_subsets, subset,
                         sens_histo=None, acf_histo=None, additive_histo=None,
                         global_scale=1.0, denom_threshold=1e-35, bins=None):
@@ -1123,6 +1137,21 @@ class OperatorProjectorDevice:
         raise RuntimeError("The Projection Data provided is not a "
                            "ProjectionList, ListModeLUT nor Histogram3D")
 
+    def _whole_histogram(self, projData, vals, p: DeviceProjector) -> bool:
+        """Whether the bins of the iterator can be projected from their index
+        (forward_histo3d): a subset of the projector's own histogram and one
+        float32 value per bin.  Other iterators, scanners and value arrays go
+        through lists of bins and crystal pairs."""
+        it, h = self.bin_iter, projData
+        return (isinstance(h, Histogram3D) and type(it) is BinIteratorRangeHistogram3D
+                and h.scanner is p.scanner
+                and (it.numZBin, it.numPhi, it.numR) == (h.numZBin, h.numPhi, h.numR)
+                and 0 <= it.idxSubset < it.numSubsets
+                and vals.is_cuda and vals.dtype == torch.float32 and vals.is_contiguous()
+                and vals.dim() == 1 and vals.numel() == h.histoSize
+                and not vals.requires_grad
+                and p.get_image_layout() == L.YRTB_LAYOUT_ROW_MAJOR)
+
     def _check_image(self, img: torch.Tensor, p: DeviceProjector):
         if not isinstance(img, torch.Tensor) or not img.is_cuda:
             raise RuntimeError("The image provided is not a CUDA tensor")
@@ -1138,6 +1167,10 @@ class OperatorProjectorDevice:
         p = self._projector()
         self._check_image(img, p)
         vals = proj._require()
+        if self._whole_histogram(proj.reference, vals, p):
+            p.forward_histo3d(img.contiguous(), vals, self.bin_iter.numSubsets,
+                              self.bin_iter.idxSubset)
+            return proj
         ev, rng = self._events(proj)
         x = img.contiguous()
         if isinstance(proj.reference, Histogram3D):
@@ -1154,6 +1187,9 @@ class OperatorProjectorDevice:
         p = self._projector()
         self._check_image(img, p)
         vals = proj._require()
+        if self._whole_histogram(proj.reference, vals, p):
+            return p.backward_histo3d(vals, img, self.bin_iter.numSubsets,
+                                      self.bin_iter.idxSubset)
         ev, rng = self._events(proj)
         if isinstance(proj.reference, Histogram3D):
             idx = torch.from_numpy(self.bin_iter.indices().astype(np.int64)).to(vals.device)
