@@ -169,3 +169,38 @@ def test_histogram_bins_refuse_what_crystal_pairs_refuse():
         op.applyA(torch.zeros(ip.shape, device="cuda"), vals)
     with pytest.raises(RuntimeError, match="requires per-event TOF values"):
         op.applyAH(vals, torch.zeros(ip.shape, device="cuda"))
+
+
+# Rows of a multiple of 4 voxels take the float4 form of the distance-driven
+# walk; images that start between 16-byte boundaries take the scalar one.
+@pytest.mark.parametrize("dims,lengths,mrd", [((40, 36, 12), (160.0, 150.0, 40.0), 4),
+                                              ((8, 9, 30), (150.0, 150.0, 60.0), 4),
+                                              ((4, 4, 3), (200.0, 200.0, 12.0), 0)])
+def test_dd_psf_histogram_quads_equal_scalar(dims, lengths, mrd):
+    sc = yrt.Scanner("t", 40, 4, 4, 10, 100, 48, 6, 1, mrd, 3, 1)
+    ip = yrt.ImageParams(*dims, *lengths)
+    pp = yrt.ProjectorParams(sc)
+    pp.setProjector("DD")
+    pp.precision = L.YRTB_COMPENSATED
+    k = np.exp(-0.5 * ((np.arange(17) - 8) * 0.6 / 1.7) ** 2)
+    taps = np.stack([k, np.roll(k, 1)]) / (k.sum() * 0.6)  # the second row is not symmetric
+    pp.setProjPsf(30.0, 0.6, taps.astype(np.float32))
+    p = yrt.DeviceProjector(sc, ip, pp)
+    h = yrt.Histogram3D(sc)
+    rng = np.random.default_rng(dims[0])
+    meas = torch.from_numpy(rng.poisson(1.0, h.histoSize).astype(np.float32)).cuda()
+    n = ip.numVoxels
+    x = torch.from_numpy(0.2 + rng.random(n + 1, np.float32)).cuda()
+
+    def em(first):
+        img = torch.empty(n + 1, device="cuda")[first:first + n].copy_(x[:n])
+        buf = torch.zeros(n + 9, device="cuda")
+        p.em_step_histo3d(img, buf[first:first + n], meas, 3, 1)
+        assert not buf[first + n:].any() and not buf[:first].any()
+        return buf[first:first + n].double()
+
+    quads, scalar = em(0), em(1)
+    assert float(scalar.norm()) > 0
+    # The weights differ by the rounding of tap coordinates counted from
+    # another voxel (2 ulp of up to 18 taps, 0.25 of a tap's weight each).
+    assert float((quads - scalar).norm() / scalar.norm()) < 3e-6

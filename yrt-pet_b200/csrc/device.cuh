@@ -49,10 +49,10 @@ struct Psf
 	const float* flipped;  // adjoint taps
 	int num_s, size;
 	float sStep, kSpacing;
-	// Prefix sums of the trapezoid bins of each kernel row (num_s * (size +
-	// 3)): prefix[m] = sum over bins xi = -1 .. m-2 of step (v(xi) + v(xi+1)) / 2.
-	const float* prefix;
-	const float* prefixFlipped;
+	// Integral of each kernel row as a piecewise parabola (num_s * (size + 2)
+	// pieces, see psfCdf), of the taps and of the flipped taps.
+	const float4* cdf;
+	const float4* cdfFlipped;
 };
 
 struct Scan
@@ -892,27 +892,22 @@ struct MultiRay
 // ---------------------------------------------------------------- DD -----
 // Integral of the linearly interpolated kernel over [x0, x1]: partial bins at
 // both ends plus the whole bins between them, summed bin by bin in the
-// reference's order, or (prefix given) as a difference of the row's prefix
-// sums, one subtraction instead of a loop over the taps.
+// reference's order.
 __device__ __forceinline__ float psfIntegral(const float* kernel,
                                              int kernelSize, float kernelStep,
-                                             float x0, float x1,
-                                             const float* prefix = nullptr,
-                                             float invStep = 0.f)
+                                             float x0, float x1)
 {
 	const int halfSize = (kernelSize - 1) / 2;
 	if (x0 > (halfSize + 1) * kernelStep || x1 < -(halfSize + 1) * kernelStep ||
 	    x0 >= x1)
 		return 0.f;
-	// The prefix form (compensated precision) scales by the reciprocal of the
-	// step; the bin-by-bin form divides as the reference does.
-	const float x0_s = prefix ? x0 * invStep : x0 / kernelStep;
+	const float x0_s = x0 / kernelStep;
 	const int x0_i = static_cast<int>(floorf(x0_s + halfSize));
 	const float tau_0 = x0_s + -(-halfSize + x0_i);
 	const float v0_lo = (x0_i < 0 || x0_i >= kernelSize) ? 0.f : __ldg(kernel + x0_i);
 	const float v0_hi = (x0_i < -1 || x0_i >= kernelSize - 1) ? 0.f : __ldg(kernel + x0_i + 1);
 	const float v0 = v0_lo * (1 - tau_0) + v0_hi * tau_0;
-	const float x1_s = prefix ? x1 * invStep : x1 / kernelStep;
+	const float x1_s = x1 / kernelStep;
 	const int x1_i = static_cast<int>(floorf(x1_s + halfSize));
 	const float tau_1 = x1_s - (-halfSize + x1_i);
 	const float v1_lo = (x1_i < 0 || x1_i >= kernelSize) ? 0.f : __ldg(kernel + x1_i);
@@ -930,32 +925,43 @@ __device__ __forceinline__ float psfIntegral(const float* kernel,
 		// Bins entirely outside [-1, kernelSize] contribute exactly zero.
 		const int xi_lo = max(x0_i + 1, -1);
 		const int xi_hi = min(x1_i, kernelSize + 1);
-		if (prefix != nullptr)
+		for (int xi = xi_lo; xi < xi_hi; xi++)
 		{
-			if (xi_hi > xi_lo)
-				out += __ldg(prefix + xi_hi + 1) - __ldg(prefix + xi_lo + 1);
-		}
-		else
-		{
-			for (int xi = xi_lo; xi < xi_hi; xi++)
-			{
-				const float v_lo = (xi < 0 || xi >= kernelSize) ? 0.f : __ldg(kernel + xi);
-				const float v_hi = (xi + 1 < 0 || xi + 1 >= kernelSize) ? 0.f : __ldg(kernel + xi + 1);
-				out += kernelStep * 0.5f * (v_lo + v_hi);
-			}
+			const float v_lo = (xi < 0 || xi >= kernelSize) ? 0.f : __ldg(kernel + xi);
+			const float v_hi = (xi + 1 < 0 || xi + 1 >= kernelSize) ? 0.f : __ldg(kernel + xi + 1);
+			out += kernelStep * 0.5f * (v_lo + v_hi);
 		}
 	}
 	return out;
 }
 
+// The integral of the same kernel as a table: the kernel is linear between its
+// taps, so its integral is a parabola on each of the size + 1 pieces between
+// them (u = 0 .. size + 1, in steps from one step before the first tap; smaller
+// and larger u are clamped), q = {value at the piece's start, first and second
+// coefficient}.  Pieces before the centre tap hold the integral from the left
+// end, pieces from it on minus the integral to the right end, so that both
+// tails keep their relative precision: the integral from a to b is cdf(b) -
+// cdf(a), plus the whole (first entry's w) if the centre lies between them.
+// (Measured from the left end throughout, the weights in the right tail lost
+// five digits, and an image whose lines see only tails was 1.2e-5 from 64 bits
+// instead of 1.7e-6.)  One 16-byte read and two fused multiply-adds, where
+// the bins' form takes about 60 instructions.  A NaN u counts as 0.
+__device__ __forceinline__ float psfCdf(const float4* __restrict__ cdf, float top, float u)
+{
+	u = fminf(fmaxf(u, 0.f), top);
+	// Integer part by an addition that rounds down into the low mantissa bits.
+	const float f = __fadd_rd(u, 8388608.f);
+	const int i = __float_as_int(f) & 0x7fffff;
+	const float t = u - (f - 8388608.f);
+	const float4 q = __ldg(cdf + i);
+	return __fmaf_rn(t, __fmaf_rn(t, q.z, q.y), q.x);
+}
+
 // Distance-driven footprint of one LOR.  d1, d2: crystal centres relative to
 // the image centre; n1, n2: crystal orientations.  visit(offset, weight).
-// FASTPSF: PSF integrals from the prefix sums (compensated precision).
-// FAST (compensated precision): every division by a value that is constant
-// along the LOR or along a row becomes a product with its reciprocal, taken
-// once (at most 1 ulp more rounding per weight); otherwise the reference's
-// divisions in its order.
-template <bool TOF, bool PSF, bool FASTPSF, bool FAST = false, typename Visit>
+// The reference's divisions in its order (ddPsfWalk is the compensated form).
+template <bool TOF, bool PSF, typename Visit>
 __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
                                        const float3 d2, const float3 n1,
                                        const float3 n2, float thickness_trans,
@@ -968,7 +974,6 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 	const bool flag_y = fabsf(d12.y) > fabsf(d12.x);
 	const float d_norm = sqrtf(d12.x * d12.x + d12.y * d12.y + d12.z * d12.z);
 	const float* kern = nullptr;
-	const float* kpre = nullptr;
 	float ext = 0.f;
 	if constexpr (PSF)
 	{
@@ -986,8 +991,6 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 			                                                    static_cast<int>(si);
 		}
 		kern = (forward ? psf.taps : psf.flipped) + s_idx * psf.size;
-		if constexpr (FASTPSF)
-			kpre = (forward ? psf.prefix : psf.prefixFlipped) + s_idx * (psf.size + 3);
 		ext = static_cast<float>((psf.size + 1) / 2) * psf.kSpacing;
 	}
 	const float dx = g.vx, dy = g.vy, dz = g.vz;
@@ -1071,13 +1074,6 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 	const float z_off = static_cast<float>(g.nz - 1) * 0.5f;
 	const float inv_dz = 1.0f / dz;
 	const float half_dyx = dyx * 0.5f;
-	// FAST: reciprocals of the denominators that are constant along the LOR.
-	const float r_xy_lo = FAST ? 1.0f / (d2_xy_hi - d1_xy_lo) : 0.f;
-	const float r_xy_hi = FAST ? 1.0f / (d2_xy_lo - d1_xy_hi) : 0.f;
-	const float r_z_lo = FAST ? 1.0f / (d2_z_lo_i - d1_z_lo_i) : 0.f;
-	const float r_z_hi = FAST ? 1.0f / (d2_z_hi_i - d1_z_hi_i) : 0.f;
-	const float r_i = (FAST && TOF) ? 1.0f / (d2_i - d1_i) : 0.f;
-	const float r_step = (FAST && PSF) ? 1.0f / psf.kSpacing : 0.f;
 
 	// Piece `part` of `parts` (several threads per LOR): an even share of the
 	// main-axis rows, each row computed exactly as by a single thread.
@@ -1091,14 +1087,10 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 	for (int xyi = row_lo; xyi <= row_hi; xyi++)
 	{
 		const float pix_xy = -0.5f * lxy + (static_cast<float>(xyi) + 0.5f) * dxy;
-		const float a_xy_lo = FAST ? (pix_xy - d1_xy_lo) * r_xy_lo
-		                           : (pix_xy - d1_xy_lo) / (d2_xy_hi - d1_xy_lo);
-		const float a_xy_hi = FAST ? (pix_xy - d1_xy_hi) * r_xy_hi
-		                           : (pix_xy - d1_xy_hi) / (d2_xy_lo - d1_xy_hi);
-		const float a_z_lo = FAST ? (pix_xy - d1_z_lo_i) * r_z_lo
-		                          : (pix_xy - d1_z_lo_i) / (d2_z_lo_i - d1_z_lo_i);
-		const float a_z_hi = FAST ? (pix_xy - d1_z_hi_i) * r_z_hi
-		                          : (pix_xy - d1_z_hi_i) / (d2_z_hi_i - d1_z_hi_i);
+		const float a_xy_lo = (pix_xy - d1_xy_lo) / (d2_xy_hi - d1_xy_lo);
+		const float a_xy_hi = (pix_xy - d1_xy_hi) / (d2_xy_lo - d1_xy_hi);
+		const float a_z_lo = (pix_xy - d1_z_lo_i) / (d2_z_lo_i - d1_z_lo_i);
+		const float a_z_hi = (pix_xy - d1_z_hi_i) / (d2_z_hi_i - d1_z_hi_i);
 		float r0 = d1_yx_lo + a_xy_lo * (d2_yx_hi - d1_yx_lo);
 		float r1 = d1_yx_hi + a_xy_hi * (d2_yx_lo - d1_yx_hi);
 		if (r0 > r1)
@@ -1127,16 +1119,10 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 		float tw = 1.f;
 		if constexpr (TOF)
 		{
-			const float a_lo = FAST ? (pix_xy - d1_i - 0.5f * dxy) * r_i
-			                        : (pix_xy - d1_i - 0.5f * dxy) / (d2_i - d1_i);
-			const float a_hi = FAST ? (pix_xy - d1_i + 0.5f * dxy) * r_i
-			                        : (pix_xy - d1_i + 0.5f * dxy) / (d2_i - d1_i);
+			const float a_lo = (pix_xy - d1_i - 0.5f * dxy) / (d2_i - d1_i);
+			const float a_hi = (pix_xy - d1_i + 0.5f * dxy) / (d2_i - d1_i);
 			tw = tofWeight(tp, d_norm, tofValue, a_lo * d_norm, a_hi * d_norm);
 		}
-		// FAST: per-row reciprocals of the footprint widths, and the
-		// row factor dxy/cos(theta) folded into the transverse weight.
-		const float r_wyx = FAST ? 1.0f / widthFrac_yx : 0.f;
-		const float r_wz = FAST ? 1.0f / widthFrac_z : 0.f;
 		// The z overlaps of the row's footprint are the same for every
 		// transverse voxel of the row: up to kDDZ of them are computed once
 		// per row (zq[j] = the factor of voxel zi0 + j, zmask its bit when the
@@ -1155,7 +1141,7 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 				const float pix_z = -0.5f * g.lz + (static_cast<float>(zi) + 0.5f) * g.vz;
 				const float zp0 = pix_z - g.vz * 0.5f, zp1 = pix_z + g.vz * 0.5f;
 				const float wz = fminf(zp1, zr1) - fmaxf(zp0, zr0);
-				zq[j] = FAST ? wz * r_wz : wz / widthFrac_z;
+				zq[j] = wz / widthFrac_z;
 				if (zi <= zi1 && zr1 >= zp0 && zr0 < zp1)
 					zmask |= 1u << j;
 			}
@@ -1171,17 +1157,17 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 			{
 				const int halfWidth = (psf.size + 1) / 2;
 				const float xa = p0 - r1_ov, xb = p1 - r0_ov;
-				if (xa > halfWidth * psf.kSpacing || xb < -halfWidth * psf.kSpacing || xa >= xb)
+				if (xa > halfWidth * psf.kSpacing || xb < -halfWidth * psf.kSpacing ||
+				         xa >= xb)
 					wxy = 0.f;
 				else
-					wxy = psfIntegral(kern, psf.size, psf.kSpacing, xa, xb,
-					                  FASTPSF ? kpre : nullptr, r_step);
+					wxy = psfIntegral(kern, psf.size, psf.kSpacing, xa, xb);
 			}
 			else
 			{
 				wxy = fminf(p1, r1_ov) - fmaxf(p0, r0_ov);
 			}
-			const float wxy_s = FAST ? wxy * r_wyx * dxy_cos_theta : wxy / widthFrac_yx;
+			const float wxy_s = wxy / widthFrac_yx;
 			const int oxy = flag_y ? g.nx * xyi + yxi : g.nx * yxi + xyi;
 			if (zfit)
 			{
@@ -1191,7 +1177,7 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 					if (zmask & (1u << j))
 					{
 						const int o = (zi0 + j) * nxy + oxy;
-						float w = FAST ? wxy_s * zq[j] : wxy_s * zq[j] * dxy_cos_theta;
+						float w = wxy_s * zq[j] * dxy_cos_theta;
 						if constexpr (TOF)
 							w *= tw;
 						visit(o, w);
@@ -1207,11 +1193,384 @@ __device__ __forceinline__ void ddWalk(const Geom& g, const float3 d1,
 				{
 					const float wz = fminf(zp1, zr1) - fmaxf(zp0, zr0);
 					const int o = zi * nxy + oxy;
-					float w = FAST ? wxy_s * (wz * r_wz)
-					               : wxy_s * (wz / widthFrac_z) * dxy_cos_theta;
+					float w = wxy_s * (wz / widthFrac_z) * dxy_cos_theta;
 					if constexpr (TOF)
 						w *= tw;
 					visit(o, w);
+				}
+			}
+		}
+	}
+}
+
+// Reciprocal in one instruction (within 1 ulp).
+__device__ __forceinline__ float rcpApprox(float x)
+{
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+	return r;
+}
+
+// Planes whose weights ddPsfWalk holds at a time.
+constexpr int kDDZ = 4;
+
+// The footprint with a projection-space PSF in compensated arithmetic.  The
+// kernel is bound by instruction issue and the latency of its image reads, so
+// the row and voxel arithmetic is kept short: divisions by what is constant
+// along the LOR or a row are products with reciprocals, the PSF integral of a
+// voxel is a difference of two tabulated values whose arguments advance by a
+// constant per voxel, and no integer <-> float conversion is made per voxel
+// (those run at an eighth of the rate of additions or less).  The weight of a voxel is separable in a
+// row, w * zq[j] for the z voxels of a column, and a whole column is handed to
+// visit(offset of its first voxel, plane stride, w, zq, mask of its voxels).
+//
+// QUADS (rows of a multiple of 4 voxels): visits are 4 consecutive x of one
+// plane instead, visit(offset, weights), so that a back projection sends one
+// float4 reduction where it sent up to 4 scalar ones: these run at 190 G/s
+// whatever their width, and the scalar form's 670 M per launch below took
+// most of it.  A line that runs along y takes the quads of each row's
+// footprint; one that runs along x takes 4 rows (x) at a time and the columns
+// of their union, where a row outside its footprint has weight 0.
+//
+// 275,000 bins of 256 x 16 crystals, 200 x 200 x 100 voxels, forward and back:
+// 8.7 ms with bin-by-bin prefix sums per voxel, 4.6 ms with columns, 3.7 ms
+// with quads (at 80 registers and 3 blocks per SM; 4.5 at 2 blocks, where the
+// columns, which wait for the L2 anyway, are as fast).
+template <bool TOF, bool QUADS, typename Visit>
+__device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const float3 d2,
+                                          const float3 n1, const float3 n2,
+                                          float thickness_trans, float thickness_z,
+                                          const TofP& tp, float tofValue, const Psf& psf,
+                                          bool forward, Visit& visit, int part = 0,
+                                          int parts = 1)
+{
+	const float3 d12 = f3sub(d1, d2);
+	const bool flag_y = fabsf(d12.y) > fabsf(d12.x);
+	const float d_norm = sqrtf(d12.x * d12.x + d12.y * d12.y + d12.z * d12.z);
+	const float4* cdf = nullptr;
+	float ext = 0.f;
+	{
+		float npx = d2.y - d1.y;
+		float npy = d1.x - d2.x;
+		const float nn = sqrtf(npx * npx + npy * npy);
+		int s_idx = 0;
+		if (nn != 0.f)
+		{
+			npx /= nn;
+			npy /= nn;
+			const float s = fabsf(d1.x * npx + d1.y * npy);
+			const float si = floorf(s / psf.sStep);
+			s_idx = (si >= static_cast<float>(psf.num_s - 1)) ? psf.num_s - 1 :
+			                                                    static_cast<int>(si);
+		}
+		cdf = (forward ? psf.cdf : psf.cdfFlipped) + s_idx * (psf.size + 2);
+		ext = static_cast<float>((psf.size + 1) / 2) * psf.kSpacing;
+	}
+	const float dx = g.vx, dy = g.vy, dz = g.vz;
+	const float inv_x = (d1.x == d2.x) ? 0.0f : 1.0f / (d2.x - d1.x);
+	const float inv_y = (d1.y == d2.y) ? 0.0f : 1.0f / (d2.y - d1.y);
+	const float inv_z = (d1.z == d2.z) ? 0.0f : 1.0f / (d2.z - d1.z);
+	float ax_min, ax_max, ay_min, ay_max, az_min, az_max;
+	slabAlpha<float>(-0.5f * (g.lx - dx), 0.5f * (g.lx - dx), d1.x, d2.x, inv_x, ax_min, ax_max);
+	slabAlpha<float>(-0.5f * (g.ly - dy), 0.5f * (g.ly - dy), d1.y, d2.y, inv_y, ay_min, ay_max);
+	slabAlpha<float>(-0.5f * (g.lz - dz), 0.5f * (g.lz - dz), d1.z, d2.z, inv_z, az_min, az_max);
+	float amin = fmaxf(fmaxf(fmaxf(0.0f, ax_min), ay_min), az_min);
+	float amax = fminf(fminf(fminf(1.0f, ax_max), ay_max), az_max);
+	if constexpr (TOF)
+	{
+		float a0, a1;
+		tofAlphaRange(tp, d_norm, tofValue, a0, a1);
+		amin = fmaxf(amin, a0);
+		amax = fminf(amax, a1);
+	}
+	const float x_0 = d1.x + amin * (d2.x - d1.x);
+	const float y_0 = d1.y + amin * (d2.y - d1.y);
+	const float x_1 = d1.x + amax * (d2.x - d1.x);
+	const float y_1 = d1.y + amax * (d2.y - d1.y);
+	const int x_i_0 = static_cast<int>(floorf(x_0 / dx + 0.5f * (g.nx - 1) + 0.5f));
+	const int y_i_0 = static_cast<int>(floorf(y_0 / dy + 0.5f * (g.ny - 1) + 0.5f));
+	const int x_i_1 = static_cast<int>(floorf(x_1 / dx + 0.5f * (g.nx - 1) + 0.5f));
+	const int y_i_1 = static_cast<int>(floorf(y_1 / dy + 0.5f * (g.ny - 1) + 0.5f));
+	const float d1_i = flag_y ? d1.y : d1.x;
+	const float d2_i = flag_y ? d2.y : d2.x;
+	const float n1_i = flag_y ? n1.y : n1.x;
+	const float n2_i = flag_y ? n2.y : n2.x;
+	const float n1_xy_norm2 = n1.x * n1.x + n1.y * n1.y;
+	const float n1_xy_norm = sqrtf(n1_xy_norm2);
+	const float n1_p_x = n1.y / n1_xy_norm;
+	const float n1_p_y = -n1.x / n1_xy_norm;
+	const float n1_z_norm = sqrtf((n1.x * n1.z) * (n1.x * n1.z) + (n1.y * n1.z) * (n1.y * n1.z) + n1_xy_norm2);
+	const float n1_p_i = (n1_i * n1.z) / n1_z_norm;
+	const float n1_p_z = -n1_xy_norm2 / n1_z_norm;
+	const float n2_xy_norm2 = n2.x * n2.x + n2.y * n2.y;
+	const float n2_xy_norm = sqrtf(n2_xy_norm2);
+	const float n2_p_x = n2.y / n2_xy_norm;
+	const float n2_p_y = -n2.x / n2_xy_norm;
+	const float n2_z_norm = sqrtf((n2.x * n2.z) * (n2.x * n2.z) + (n2.y * n2.z) * (n2.y * n2.z) + n2_xy_norm2);
+	const float n2_p_i = (n2_i * n2.z) / n2_z_norm;
+	const float n2_p_z = -n2_xy_norm2 / n2_z_norm;
+	const float htt = thickness_trans * 0.5f;
+	const float d1_xy_lo_x = d1.x - htt * n1_p_x, d1_xy_lo_y = d1.y - htt * n1_p_y;
+	const float d1_xy_hi_x = d1.x + htt * n1_p_x, d1_xy_hi_y = d1.y + htt * n1_p_y;
+	const float d2_xy_lo_x = d2.x - htt * n2_p_x, d2_xy_lo_y = d2.y - htt * n2_p_y;
+	const float d2_xy_hi_x = d2.x + htt * n2_p_x, d2_xy_hi_y = d2.y + htt * n2_p_y;
+	const float htz = thickness_z * 0.5f;
+	const float d1_z_lo_i = d1_i - htz * n1_p_i, d1_z_lo_z = d1.z - htz * n1_p_z;
+	const float d1_z_hi_i = d1_i + htz * n1_p_i, d1_z_hi_z = d1.z + htz * n1_p_z;
+	const float d2_z_lo_i = d2_i - htz * n2_p_i, d2_z_lo_z = d2.z - htz * n2_p_z;
+	const float d2_z_hi_i = d2_i + htz * n2_p_i, d2_z_hi_z = d2.z + htz * n2_p_z;
+
+	int xy_i_0, xy_i_1, nyx;
+	float lxy, lyx, dxy, dyx;
+	float d1_xy_lo, d1_xy_hi, d2_xy_lo, d2_xy_hi, d1_yx_lo, d1_yx_hi, d2_yx_lo, d2_yx_hi;
+	if (flag_y)
+	{
+		xy_i_0 = max(0, min(y_i_0, y_i_1));
+		xy_i_1 = min(g.ny - 1, max(y_i_0, y_i_1));
+		lxy = g.ly; dxy = g.vy; lyx = g.lx; dyx = g.vx; nyx = g.nx;
+		d1_xy_lo = d1_xy_lo_y; d1_xy_hi = d1_xy_hi_y; d2_xy_lo = d2_xy_lo_y; d2_xy_hi = d2_xy_hi_y;
+		d1_yx_lo = d1_xy_lo_x; d1_yx_hi = d1_xy_hi_x; d2_yx_lo = d2_xy_lo_x; d2_yx_hi = d2_xy_hi_x;
+	}
+	else
+	{
+		xy_i_0 = max(0, min(x_i_0, x_i_1));
+		xy_i_1 = min(g.nx - 1, max(x_i_0, x_i_1));
+		lxy = g.lx; dxy = g.vx; lyx = g.ly; dyx = g.vy; nyx = g.ny;
+		d1_xy_lo = d1_xy_lo_x; d1_xy_hi = d1_xy_hi_x; d2_xy_lo = d2_xy_lo_x; d2_xy_hi = d2_xy_hi_x;
+		d1_yx_lo = d1_xy_lo_y; d1_yx_hi = d1_xy_hi_y; d2_yx_lo = d2_xy_lo_y; d2_yx_hi = d2_xy_hi_y;
+	}
+	const float dxy_cos_theta =
+	    (d1_i != d2_i) ? dxy / (fabsf(d1_i - d2_i) / d_norm) : dxy;
+	const int nxy = g.nx * g.ny;
+	const float yx_off = static_cast<float>(nyx - 1) / 2.f;
+	const float inv_dyx = 1.0f / dyx;
+	const float z_off = static_cast<float>(g.nz - 1) * 0.5f;
+	const float inv_dz = 1.0f / dz;
+
+	// Piece `part` of `parts` (several threads per LOR): an even share of the
+	// main-axis rows, each row computed exactly as by a single thread.
+	int row_lo = xy_i_0, row_hi = xy_i_1;
+	if (parts > 1 && xy_i_1 >= xy_i_0)
+	{
+		const int nrows = xy_i_1 - xy_i_0 + 1;
+		row_lo = xy_i_0 + (nrows * part) / parts;
+		row_hi = xy_i_0 + (nrows * (part + 1)) / parts - 1;
+	}
+	// Reciprocals of the denominators that are constant along the LOR.
+	const float r_xy_lo = 1.0f / (d2_xy_hi - d1_xy_lo);
+	const float r_xy_hi = 1.0f / (d2_xy_lo - d1_xy_hi);
+	const float r_z_lo = 1.0f / (d2_z_lo_i - d1_z_lo_i);
+	const float r_z_hi = 1.0f / (d2_z_hi_i - d1_z_hi_i);
+	const float r_i = TOF ? 1.0f / (d2_i - d1_i) : 0.f;
+	const float r_step = 1.0f / psf.kSpacing;
+	const float top = static_cast<float>(psf.size + 1);
+	const float mid = static_cast<float>((psf.size + 1) / 2);
+	const float du = dyx * r_step;  // taps per voxel
+	const float whole = __ldg(cdf).w;
+	const float y0 = -0.5f * lyx, z0 = -0.5f * g.lz;
+	// Footprint of row xyi: transverse and axial edges, and the voxels they span
+	// (false if none).
+	struct Row
+	{
+		float r0, r1, z0, z1;
+		int i0, i1, zi0, zi1;
+	};
+	auto footprint = [&](float rowF, Row& R) -> bool
+	{
+		const float pix_xy = -0.5f * lxy + (rowF + 0.5f) * dxy;
+		const float a = d1_yx_lo + (pix_xy - d1_xy_lo) * r_xy_lo * (d2_yx_hi - d1_yx_lo);
+		const float b = d1_yx_hi + (pix_xy - d1_xy_hi) * r_xy_hi * (d2_yx_lo - d1_yx_hi);
+		const float c = d1_z_lo_z + (pix_xy - d1_z_lo_i) * r_z_lo * (d2_z_lo_z - d1_z_lo_z);
+		const float d = d1_z_hi_z + (pix_xy - d1_z_hi_i) * r_z_hi * (d2_z_hi_z - d1_z_hi_z);
+		R.r0 = fminf(a, b);
+		R.r1 = fmaxf(a, b);
+		R.z0 = fminf(c, d);
+		R.z1 = fmaxf(c, d);
+		R.i0 = max(0, __float2int_rn((R.r0 - ext) * inv_dyx + yx_off));
+		R.i1 = min(nyx - 1, __float2int_rn((R.r1 + ext) * inv_dyx + yx_off));
+		R.zi0 = max(0, __float2int_rn(R.z0 * inv_dz + z_off));
+		R.zi1 = min(g.nz - 1, __float2int_rn(R.z1 * inv_dz + z_off));
+		// (r0 <= r1 and z0 <= z1 unless an edge is not a number.)
+		return R.i0 <= R.i1 && R.zi0 <= R.zi1 && R.r0 <= R.r1 && R.z0 <= R.z1;
+	};
+	// Row factor of the transverse weights.
+	auto rowWeight = [&](float rowF, const Row& R) -> float
+	{
+		float w = rcpApprox(R.r1 - R.r0) * dxy_cos_theta;
+		if constexpr (TOF)
+		{
+			const float pix_xy = -0.5f * lxy + (rowF + 0.5f) * dxy;
+			const float a_lo = (pix_xy - d1_i - 0.5f * dxy) * r_i;
+			const float a_hi = (pix_xy - d1_i + 0.5f * dxy) * r_i;
+			w *= tofWeight(tp, d_norm, tofValue, a_lo * d_norm, a_hi * d_norm);
+		}
+		return w;
+	};
+	// Integral of the kernel over a voxel, from the tap coordinates of its
+	// near edge from the footprint's far end (ua) and of its far edge from the
+	// near end (ub); 0 outside the support.
+	auto integral = [&](float ua, float ub) -> float
+	{
+		const float w = psfCdf(cdf, top, ub) - psfCdf(cdf, top, ua);
+		return (ua < mid && ub >= mid) ? w + whole : w;
+	};
+	// Overlap of plane z0 + (zf + j) dz .. with an axial footprint, as a
+	// fraction of its width (0 if they don't meet).
+	auto axial = [&](float zf, int j, float lo, float hi, float inv) -> float
+	{
+		const float p0 = z0 + (zf + static_cast<float>(j)) * dz, p1 = p0 + dz;
+		return (hi >= p0 && lo < p1) ? (fminf(p1, hi) - fmaxf(p0, lo)) * inv : 0.f;
+	};
+
+	if constexpr (QUADS)
+	{
+		if (flag_y)
+		{
+			for (int xyi = row_lo; xyi <= row_hi; xyi++)
+			{
+				const float rowF = static_cast<float>(xyi);
+				Row R;
+				if (!footprint(rowF, R))
+					continue;
+				const float rowW = rowWeight(rowF, R), r_wz = rcpApprox(R.z1 - R.z0);
+				const int q0 = R.i0 & ~3;
+				const float edge = y0 + static_cast<float>(q0) * dyx;
+				const float ua0 = __fmaf_rn(edge - R.r1, r_step, mid);
+				const float ub0 = __fmaf_rn(edge + dyx - R.r0, r_step, mid);
+				for (int zi = R.zi0; zi <= R.zi1; zi += kDDZ)
+				{
+					float zq[kDDZ];
+					const float zf = static_cast<float>(zi);
+#pragma unroll
+					for (int j = 0; j < kDDZ; j++)
+						zq[j] = zi + j <= R.zi1 ? axial(zf, j, R.z0, R.z1, r_wz) : 0.f;
+					int o = zi * nxy + xyi * g.nx + q0;
+					float kf = 0.f;
+					for (int x = q0; x <= R.i1; x += 4, kf += 4.f, o += 4)
+					{
+						float w[4];
+#pragma unroll
+						for (int l = 0; l < 4; l++)
+						{
+							const float k = kf + static_cast<float>(l);
+							const float ua = __fmaf_rn(k, du, ua0), ub = __fmaf_rn(k, du, ub0);
+							w[l] = integral(ua, ub) * rowW;
+						}
+#pragma unroll
+						for (int j = 0; j < kDDZ; j++)
+							if (zq[j] != 0.f)
+								visit(o + j * nxy, make_float4(w[0] * zq[j], w[1] * zq[j],
+								                               w[2] * zq[j], w[3] * zq[j]));
+					}
+				}
+			}
+		}
+		else
+		{
+			// Quads of rows; each part takes an even share of all of them.
+			const int qlo = xy_i_0 >> 2, nq = (xy_i_1 >> 2) - qlo + 1;
+			const int qa = xy_i_1 >= xy_i_0 ? qlo + nq * part / parts : 0;
+			const int qb = xy_i_1 >= xy_i_0 ? qlo + nq * (part + 1) / parts : 0;
+			for (int q = qa; q < qb; q++)
+			{
+				// A row without a footprint: weight and overlaps 0.
+				float rw[4], rz[4], ra[4], rb[4], z0q[4], z1q[4];
+				int ilo = nyx, ihi = -1, zlo = g.nz, zhi = -1;
+#pragma unroll
+				for (int l = 0; l < 4; l++)
+				{
+					const int xyi = 4 * q + l;
+					const float rowF = static_cast<float>(xyi);
+					Row R;
+					const bool ok = xyi >= xy_i_0 && xyi <= xy_i_1 && footprint(rowF, R);
+					rw[l] = ok ? rowWeight(rowF, R) : 0.f;
+					rz[l] = ok ? rcpApprox(R.z1 - R.z0) : 0.f;
+					ra[l] = ok ? R.r0 : 0.f;
+					rb[l] = ok ? R.r1 : 0.f;
+					z0q[l] = ok ? R.z0 : 3.0e38f;
+					z1q[l] = ok ? R.z1 : -3.0e38f;
+					if (ok)
+					{
+						ilo = min(ilo, R.i0);
+						ihi = max(ihi, R.i1);
+						zlo = min(zlo, R.zi0);
+						zhi = max(zhi, R.zi1);
+					}
+				}
+				const float edge = y0 + static_cast<float>(ilo) * dyx;
+				float ua0[4], ub0[4];
+#pragma unroll
+				for (int l = 0; l < 4; l++)
+				{
+					ua0[l] = __fmaf_rn(edge - rb[l], r_step, mid);
+					ub0[l] = __fmaf_rn(edge + dyx - ra[l], r_step, mid);
+				}
+				for (int zi = zlo; zi <= zhi; zi += kDDZ)
+				{
+					float zq[4][kDDZ];
+					const float zf = static_cast<float>(zi);
+#pragma unroll
+					for (int j = 0; j < kDDZ; j++)
+#pragma unroll
+						for (int l = 0; l < 4; l++)
+							zq[l][j] = axial(zf, j, z0q[l], z1q[l], rz[l]);
+					int o = zi * nxy + ilo * g.nx + 4 * q;
+					float kf = 0.f;
+					for (int yxi = ilo; yxi <= ihi; yxi++, kf += 1.f, o += g.nx)
+					{
+						float w[4];
+#pragma unroll
+						for (int l = 0; l < 4; l++)
+						{
+							const float ua = __fmaf_rn(kf, du, ua0[l]);
+							const float ub = __fmaf_rn(kf, du, ub0[l]);
+							w[l] = integral(ua, ub) * rw[l];
+						}
+#pragma unroll
+						for (int j = 0; j < kDDZ; j++)
+							if (zi + j <= zhi)
+								visit(o + j * nxy, make_float4(w[0] * zq[0][j], w[1] * zq[1][j],
+								                               w[2] * zq[2][j], w[3] * zq[3][j]));
+					}
+				}
+			}
+		}
+	}
+	else
+	{
+		const int sxy = flag_y ? g.nx : 1, syx = flag_y ? 1 : g.nx;
+		for (int xyi = row_lo; xyi <= row_hi; xyi++)
+		{
+			const float rowF = static_cast<float>(xyi);
+			Row R;
+			if (!footprint(rowF, R))
+				continue;
+			const float rowW = rowWeight(rowF, R), r_wz = rcpApprox(R.z1 - R.z0);
+			const float edge = y0 + static_cast<float>(R.i0) * dyx;
+			const float ua0 = __fmaf_rn(edge - R.r1, r_step, mid);
+			const float ub0 = __fmaf_rn(edge + dyx - R.r0, r_step, mid);
+			const int rowO = xyi * sxy + R.i0 * syx;
+			for (int zi = R.zi0; zi <= R.zi1; zi += kDDZ)
+			{
+				float zq[kDDZ];
+				unsigned zmask = 0u;
+				const float zf = static_cast<float>(zi);
+#pragma unroll
+				for (int j = 0; j < kDDZ; j++)
+				{
+					const float zp0 = z0 + (zf + static_cast<float>(j)) * dz;
+					zq[j] = axial(zf, j, R.z0, R.z1, r_wz);
+					if (zi + j <= R.zi1 && R.z1 >= zp0 && R.z0 < zp0 + dz)
+						zmask |= 1u << j;
+				}
+				int o = zi * nxy + rowO;
+				float kf = 0.f;
+				for (int yxi = R.i0; yxi <= R.i1; yxi++, kf += 1.f, o += syx)
+				{
+					const float ua = __fmaf_rn(kf, du, ua0), ub = __fmaf_rn(kf, du, ub0);
+					if (!(ua <= top && ub > 0.f))
+						continue;
+					visit(o, nxy, integral(ua, ub) * rowW, zq, zmask);
 				}
 			}
 		}

@@ -466,9 +466,32 @@ __device__ __forceinline__ void projectEvent(const KParams& P, float3 p1,
 	}
 	else
 	{
-		ddWalk<TOF, KIND == K_DD_PSF, COMP && KIND == K_DD_PSF, COMP>(P.g, p1, p2, n1, n2, P.scan.crystalTrans,
-		                              P.scan.crystalZ, P.tof, tofv, P.psf,
-		                              forward, visit, part, parts);
+		constexpr bool kQuads = std::is_invocable_v<Visit&, int, float4>;
+		constexpr bool kColumns =
+		    std::is_invocable_v<Visit&, int, int, float, const float(&)[kDDZ], unsigned>;
+		if constexpr (KIND == K_DD_PSF && COMP && (kColumns || kQuads))
+		{
+			ddPsfWalk<TOF, kQuads>(P.g, p1, p2, n1, n2, P.scan.crystalTrans, P.scan.crystalZ, P.tof, tofv,
+			               P.psf, forward, visit, part, parts);
+		}
+		else if constexpr (KIND == K_DD_PSF && COMP)
+		{
+			auto column = [&](int o, int stride, float w, const float(&zq)[kDDZ], unsigned mask)
+			{
+#pragma unroll
+				for (int j = 0; j < kDDZ; j++)
+					if (mask & (1u << j))
+						visit(o + j * stride, w * zq[j]);
+			};
+			ddPsfWalk<TOF, false>(P.g, p1, p2, n1, n2, P.scan.crystalTrans, P.scan.crystalZ,
+			                      P.tof, tofv, P.psf, forward, column, part, parts);
+		}
+		else
+		{
+			ddWalk<TOF, KIND == K_DD_PSF>(P.g, p1, p2, n1, n2, P.scan.crystalTrans,
+			                              P.scan.crystalZ, P.tof, tofv, P.psf, forward, visit,
+			                              part, parts);
+		}
 		endRay();
 	}
 }
@@ -534,8 +557,57 @@ __device__ __forceinline__ float forwardEvent(const KParams& P,
 		ray = 0.f;
 		comp = 0.f;
 	};
-	projectEvent<KIND, TOF, COMP, TILE, WARP>(P, p1, p2, n1, n2, tofv, rid, true, visit,
-	                                          endRay, part, parts, alive);
+	if constexpr (KIND == K_DD_PSF && COMP && VEC)
+	{
+		// Voxels outside the footprint (weight 0) are read but not used.
+		auto quad = [&](int o, float4 w)
+		{
+			const float4 q = __ldg(reinterpret_cast<const float4*>(img + o));
+			float c = w.x != 0.f ? w.x * q.x : 0.f;
+			c = w.y != 0.f ? __fmaf_rn(w.y, q.y, c) : c;
+			c = w.z != 0.f ? __fmaf_rn(w.z, q.z, c) : c;
+			c = w.w != 0.f ? __fmaf_rn(w.w, q.w, c) : c;
+			const float y = c - comp;
+			const float t = ray + y;
+			comp = (t - ray) - y;
+			ray = t;
+		};
+		projectEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2, tofv, rid, true, quad, endRay, part,
+		                              parts);
+	}
+	else if constexpr (KIND == K_DD_PSF && COMP)
+	{
+		// A column's products are summed before they enter the compensated
+		// sum: its reads are in flight together.
+		auto column = [&](int o, int stride, float w, const float(&zq)[kDDZ], unsigned mask)
+		{
+			float q[kDDZ], c = 0.f;
+#pragma unroll
+			for (int j = 0; j < kDDZ; j++)
+				q[j] = (mask & (1u << j)) ? __ldg(img + o + j * stride) : 0.f;
+#pragma unroll
+			for (int j = 0; j < kDDZ; j++)
+			{
+				if (mask & (1u << j))
+				{
+					c = __fmaf_rn(zq[j], q[j], c);
+					if constexpr (TRACK)
+						mw = fmaxf(mw, fabsf(w * zq[j]));
+				}
+			}
+			const float y = __fmaf_rn(w, c, -comp);
+			const float t = ray + y;
+			comp = (t - ray) - y;
+			ray = t;
+		};
+		projectEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2, tofv, rid, true, column, endRay, part,
+		                              parts);
+	}
+	else
+	{
+		projectEvent<KIND, TOF, COMP, TILE, WARP>(P, p1, p2, n1, n2, tofv, rid, true, visit,
+		                                          endRay, part, parts, alive);
+	}
 	// One lane per ray (parts > 1): the caller adds the rays' sums in ray
 	// order and divides (rayGroupMean).
 	if constexpr (KIND == K_SIDDON_MR)
@@ -1412,7 +1484,7 @@ struct HistoArgs
 
 // Blocks per SM of the compensated DD + PSF histogram EM kernel (several
 // threads per bin).
-constexpr int kDDPsfBlocksPerSM = 2;
+constexpr int kDDPsfBlocksPerSM = 3;
 
 // Item t (ok: it exists) of a histogram operation: subset-local bin t, or
 // list[t] with a list (which then holds only the bins that do work).
@@ -1422,7 +1494,8 @@ constexpr int kDDPsfBlocksPerSM = 2;
 // step, so every lane of a warp calls this: the bins of a warp are neighbours
 // in r, whose rays run side by side but step along different axes at
 // different times, and walked freely they drift apart.
-template <int KIND, int HOP, int MODE, bool COMP, int TPL>
+// QUADS: DD + PSF on float4 groups of the image (ddPsfWalk).
+template <int KIND, int HOP, int MODE, bool COMP, int TPL, bool QUADS = false>
 __device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, const HistoArgs& A,
                                           uint64_t t, bool ok, int part)
 {
@@ -1512,7 +1585,7 @@ __device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, cons
 	{
 		float mw = 0.f, u = 0.f;
 		if (WARP || ok)
-			u = forwardEvent<KIND, false, COMP, MODE == H_BOUND, false, false, WARP>(
+			u = forwardEvent<KIND, false, COMP, MODE == H_BOUND, QUADS, false, WARP>(
 			    P, A.img, p1, p2, n1, n2, 0.f, k, MODE == H_BOUND ? &mw : nullptr, part, TPL, ok);
 		if constexpr (TPL > 1)
 			if (ok)  // the lanes of a group share the bin
@@ -1565,19 +1638,20 @@ __device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, cons
 	else
 	{
 		if (WARP || ok)
-			backwardEvent<KIND, false, COMP, false, 0, false, WARP>(
+			backwardEvent<KIND, false, COMP, false, QUADS ? 1 : 0, false, WARP>(
 			    P, A.out, v, p1, p2, n1, n2, 0.f, k, nullptr, 0.0, part, TPL, nullptr, 0, ok);
 	}
 }
 
 // One item per TPL threads: a warp's threads stay converged across items (a
 // grid-stride loop lets them drift apart between items).
-template <int KIND, int HOP, int MODE = H_PLAIN, bool COMP = false, int TPL = 1>
+template <int KIND, int HOP, int MODE = H_PLAIN, bool COMP = false, int TPL = 1,
+          bool QUADS = false>
 __global__ void __launch_bounds__(kBlock, (KIND == K_DD_PSF && TPL > 1) ? kDDPsfBlocksPerSM : 1)
     k_histo(KParams P, H3Dev H, const __grid_constant__ HistoArgs A)
 {
 	const uint64_t gt = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-	histoItem<KIND, HOP, MODE, COMP, TPL>(P, H, A, gt / TPL, gt / TPL < A.count,
+	histoItem<KIND, HOP, MODE, COMP, TPL, QUADS>(P, H, A, gt / TPL, gt / TPL < A.count,
 	                                             static_cast<int>(gt % TPL));
 }
 
@@ -2828,8 +2902,8 @@ struct yrtb_projector
 	float4* d_ori = nullptr;
 	float* d_taps = nullptr;
 	float* d_flipped = nullptr;
-	float* d_prefix = nullptr;
-	float* d_prefixFlipped = nullptr;
+	float4* d_cdf = nullptr;
+	float4* d_cdfFlipped = nullptr;
 	int32_t* d_ring = nullptr;
 	int2* d_z = nullptr;
 	unsigned long long* d_err = nullptr;
@@ -2991,7 +3065,7 @@ yrtb_status checkEvents(const yrtb_projector* h, const yrtb_events* ev,
 
 // Calls fn(kind, tof, comp) with the projector's configuration as
 // std::integral_constant / bool_constant values (compensated arithmetic
-// exists for the Siddon projectors and, as prefix-sum PSF integrals and
+// exists for the Siddon projectors and, as tabulated PSF integrals and
 // products with reciprocals of the LOR's and rows' constant denominators, for
 // distance-driven projection with a PSF).
 template <typename Fn>
@@ -3343,8 +3417,14 @@ yrtb_status dispatchHisto(yrtb_projector* h, int numSubsets, int subset, HistoAr
 			// Compensated DD + PSF EM: kHistoDDThreads threads per bin, each
 			// on an even share of the bin's rows.
 			constexpr int T = kHistoDDThreads;
-			k_histo<K, HOP, H_PLAIN, C, T><<<gridAll(A.count * T), kBlock, 0, st>>>(h->P, h->h3d,
-			                                                                       A);
+			// Quads need rows of a multiple of 4 voxels and 16-byte aligned
+			// images.
+			const bool quads = h->P.g.nx % 4 == 0 &&
+			                   reinterpret_cast<uintptr_t>(A.img) % 16 == 0 &&
+			                   reinterpret_cast<uintptr_t>(A.out) % 16 == 0;
+			auto kernel = quads ? k_histo<K, HOP, H_PLAIN, C, T, true>
+			                    : k_histo<K, HOP, H_PLAIN, C, T, false>;
+			kernel<<<gridAll(A.count * T), kBlock, 0, st>>>(h->P, h->h3d, A);
 		}
 		else
 		{
@@ -3708,34 +3788,47 @@ yrtb_status yrtb_projector_create(const yrtb_scanner* s, const float* lut,
 		YRTB_CUDA(h->make(&h->d_flipped, n));
 		YRTB_CUDA(cudaMemcpy(h->d_taps, pp->psf_taps, n * sizeof(float), cudaMemcpyHostToDevice));
 		YRTB_CUDA(cudaMemcpy(h->d_flipped, flipped.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-		// Prefix sums of the trapezoid bins per kernel row (FP64, stored FP32).
-		const int K = pp->psf_size, W = K + 3;
-		auto prefixOf = [&](const std::vector<float>& t, std::vector<float>& out)
+		// Pieces of the integral of each kernel row (psfCdf; FP64, stored
+		// FP32): piece i runs from tap i - 1 to tap i, taps beyond the ends
+		// are 0.
+		const int K = pp->psf_size, W = K + 2;
+		auto cdfOf = [&](const std::vector<float>& t)
 		{
-			out.assign(static_cast<size_t>(pp->psf_num_s) * W, 0.f);
+			std::vector<float4> out(static_cast<size_t>(pp->psf_num_s) * W);
+			const double step = pp->psf_k_spacing;
 			for (int i = 0; i < pp->psf_num_s; i++)
 			{
 				auto v = [&](int k) { return (k < 0 || k >= K) ? 0.0 : double(t[size_t(i) * K + k]); };
+				double whole = 0.0;
+				for (int k = 0; k < K; k++)
+					whole += step * v(k);
 				double acc = 0.0;
-				out[size_t(i) * W + 0] = 0.f;
-				for (int m = 1; m < W; m++)
+				for (int m = 0; m < W; m++)
 				{
-					const int xi = m - 2;
-					if (xi >= -1)
-						acc += double(pp->psf_k_spacing) * 0.5 * (v(xi) + v(xi + 1));
-					out[size_t(i) * W + m] = static_cast<float>(acc);
+					if (m == (K + 1) / 2)
+					{
+						// From the centre tap on, minus what is left of it.
+						acc = 0.0;
+						for (int k = m; k <= K; k++)
+							acc -= 0.5 * step * (v(k - 1) + v(k));
+					}
+					out[size_t(i) * W + m] =
+					    make_float4(static_cast<float>(acc), static_cast<float>(step * v(m - 1)),
+					                static_cast<float>(0.5 * step * (v(m) - v(m - 1))), 0.f);
+					acc += 0.5 * step * (v(m - 1) + v(m));
 				}
+				out[size_t(i) * W].w = static_cast<float>(whole);
 			}
+			return out;
 		};
-		std::vector<float> taps(pp->psf_taps, pp->psf_taps + n), pre, preF;
-		prefixOf(taps, pre);
-		prefixOf(flipped, preF);
-		YRTB_CUDA(h->make(&h->d_prefix, pre.size()));
-		YRTB_CUDA(h->make(&h->d_prefixFlipped, preF.size()));
-		YRTB_CUDA(cudaMemcpy(h->d_prefix, pre.data(), pre.size() * sizeof(float), cudaMemcpyHostToDevice));
-		YRTB_CUDA(cudaMemcpy(h->d_prefixFlipped, preF.data(), preF.size() * sizeof(float), cudaMemcpyHostToDevice));
+		std::vector<float> taps(pp->psf_taps, pp->psf_taps + n);
+		const std::vector<float4> cdf = cdfOf(taps), cdfF = cdfOf(flipped);
+		YRTB_CUDA(h->make(&h->d_cdf, cdf.size()));
+		YRTB_CUDA(h->make(&h->d_cdfFlipped, cdfF.size()));
+		YRTB_CUDA(cudaMemcpy(h->d_cdf, cdf.data(), cdf.size() * sizeof(float4), cudaMemcpyHostToDevice));
+		YRTB_CUDA(cudaMemcpy(h->d_cdfFlipped, cdfF.data(), cdfF.size() * sizeof(float4), cudaMemcpyHostToDevice));
 		P.psf = Psf{h->d_taps, h->d_flipped, pp->psf_num_s, pp->psf_size,
-		            pp->psf_s_step, pp->psf_k_spacing, h->d_prefix, h->d_prefixFlipped};
+		            pp->psf_s_step, pp->psf_k_spacing, h->d_cdf, h->d_cdfFlipped};
 	}
 	h->h3d.numDets = static_cast<uint32_t>(nd);
 	if (s->dets_per_ring % 2 == 0)
