@@ -176,7 +176,8 @@ void yrtb_projector_destroy(yrtb_projector* h);
  * yrtb_backward, yrtb_em_step and the OSEM driver) and of the event ordering.
  * No reference counterpart: the reference launches one thread per event in
  * 256-thread blocks (GPUBatchSetup, include/yrt-pet/utils/GPUTypes.cuh:17-55)
- * on events in file order.  Default: {256, 1, 3, YRTB_ORDER_LOR, 1, 2}. */
+ * on events in file order.  Default: {256, 1, 3, order, 1, 2}, the order
+ * YRTB_ORDER_SPATIAL for single-ray Siddon with TOF, else YRTB_ORDER_LOR. */
 #define YRTB_ORDER_LOR 0      /* inside a ray-length bucket: by LOR (Histogram3D bin), then TOF */
 #define YRTB_ORDER_SPATIAL 1  /* inside a ray-length bucket: by direction sector (16 azimuthal x
                                  2 axial), then the Morton code of the TOF kernel centre (the

@@ -231,3 +231,46 @@ def test_vector_reductions_on_ragged_images(precision, dims):
         # The same FP32 terms in two orders, at most all of them in one
         # voxel: half an ulp per addition, at random, on each side.
         assert rel_l2(back(groups), scalar) < 2 * len(d1) ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("order", [L.YRTB_ORDER_LOR, L.YRTB_ORDER_SPATIAL,
+                                   L.YRTB_ORDER_SPATIAL_FINE])
+def test_order_with_frames_groups_subsets_then_frames(order):
+    sc, _, _ = make()
+    nt, S = 5, 6
+    ip = yrt.ImageParams(*IP_ARGS, nt=nt)
+    p = yrt.DeviceProjector(sc, ip, yrt.ProjectorParams(sc))
+    p.set_launch(256, 1, 3, order=order)
+    d1, d2 = random_events(30001, 52)
+    fr = np.random.default_rng(53).integers(-2, nt + 2, len(d1)).astype(np.int32)
+    ev = yrt.DeviceEvents.from_arrays(d1, d2, frame=fr)
+    out, offs = p.order_events(ev, S, first_global_index=4)
+    perm = out.perm.cpu().numpy()
+    assert np.array_equal(np.sort(perm), np.arange(len(d1)))
+    of = out.frame.cpu().numpy()
+    assert np.array_equal(of, fr[perm])
+    for s in range(S):
+        part = slice(int(offs[s]), int(offs[s + 1]))
+        assert np.all((perm[part] + 4) % S == s)
+        f = of[part].astype(np.int64)
+        f[(f < 0) | (f >= nt)] = nt  # events without a frame come last
+        assert np.all(np.diff(f) >= 0)
+
+
+def test_multi_ray_order_is_by_subset_bin_and_tof():
+    """The offsets of an event's extra rays follow its place in the order, so
+    the order itself is part of a multi-ray result: subset, Histogram3D bin,
+    TOF in steps of 16 ps, then file order."""
+    sc = yrt.Scanner("t", *SC_ARGS)
+    pp = yrt.ProjectorParams(sc)
+    pp.numRays = 3
+    pp.addTOF(214.0, 5)
+    p = yrt.DeviceProjector(sc, yrt.ImageParams(*IP_ARGS), pp)
+    d1, d2 = random_events(20000, 61)
+    tv = np.random.default_rng(62).normal(0, 300, len(d1)).astype(np.float32)
+    S = 5
+    out, _ = p.order_events(yrt.DeviceEvents.from_arrays(d1, d2, tof=tv), S)
+    bins = yrt.histo3d_bins(sc, d1, d2).astype(np.int64)
+    q = np.clip(np.floor(tv / np.float32(16) + np.float32(128)), 0, 255).astype(np.int64)
+    want = np.lexsort((np.arange(len(d1)), q, bins, np.arange(len(d1)) % S))
+    assert np.array_equal(out.perm.cpu().numpy(), want)
