@@ -274,3 +274,47 @@ def test_multi_ray_order_is_by_subset_bin_and_tof():
     q = np.clip(np.floor(tv / np.float32(16) + np.float32(128)), 0, 255).astype(np.int64)
     want = np.lexsort((np.arange(len(d1)), q, bins, np.arange(len(d1)) % S))
     assert np.array_equal(out.perm.cpu().numpy(), want)
+
+
+# Launches at and around the largest of the small form, with skipped events, a
+# range that strides, frames, and every array of the EM pass: the same values as
+# the launch shape set by the caller.
+@pytest.mark.parametrize("precision", [L.YRTB_MIRROR, L.YRTB_COMPENSATED])
+@pytest.mark.parametrize("tof", [None, (214.0, 5)])
+@pytest.mark.parametrize("n", [1, 33, 4001, 32768, 32769, 131072, 131073])
+def test_small_launches_equal_the_set_shape(precision, tof, n):
+    sc = yrt.Scanner("t", *SC_ARGS)
+    ip = yrt.ImageParams(37, 41, 15, 128, 128, 64, nt=2)
+    pp = yrt.ProjectorParams(sc)
+    pp.precision = precision
+    if tof:
+        pp.addTOF(*tof)
+    rng = np.random.default_rng(n)
+    d1, d2 = random_events(3 * n + 8, 60)
+    m = 3 * n + 2
+    d1, d2 = np.resize(d1, m), np.resize(d2, m)
+    d1[5 % m] = 1 << 30  # no such crystal
+    f32 = lambda lo, hi: rng.uniform(lo, hi, m).astype(np.float32)
+    meas = rng.integers(0, 3, m).astype(np.float32)
+    ev = yrt.DeviceEvents.from_arrays(
+        d1, d2, tof=f32(-300, 300) if tof else None,
+        frame=rng.integers(-1, 3, m).astype(np.int32), measurement=meas, sens=f32(0.5, 1.5),
+        att=f32(0.2, 1), additive=f32(0.1, 0.2))
+    r = L.yrtb_range(2, 3, n)
+    x = torch.from_numpy(rng.random(ip.shape, np.float32)).cuda()
+    y = torch.from_numpy(f32(0, 1)).cuda()
+    out = {}
+    for shape in ("default", "set"):
+        p = yrt.DeviceProjector(sc, ip, pp)
+        if shape == "set":
+            p.set_launch(256, 1, 3, vector_groups=0)
+        fwd = p.forward(x, ev, out=torch.full((m,), -3.0, device="cuda"), rng=r)
+        bwd = p.backward(y, ev, rng=r)
+        em, model = torch.zeros_like(x), torch.full((m,), -3.0, device="cuda")
+        p.em_step(x, em, ev, rng=r, global_scale=0.7, model=model)
+        out[shape] = (fwd, model, bwd, em, p.take_event_errors())
+    a, b = out["default"], out["set"]
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    assert a[4] == b[4]
+    for i in (2, 3):  # the same terms, added in another order
+        assert rel_l2(a[i].cpu().numpy(), b[i].cpu().numpy()) < 2 * n ** 0.5 * 2.0 ** -24

@@ -1066,6 +1066,112 @@ __global__ void __launch_bounds__(BLOCK, ((KIND == K_SIDDON && COMP) ||
 	}
 }
 
+// Small launches of the single-ray Siddon operations: too few rays to hide the
+// latency of their image reads, so a walk records 8 crossings, issues their
+// reads together and adds them in walk order (the same sums as k_events), and
+// blocks of one warp spread over all SMs.  Reductions are sent per voxel: the
+// L2 has room, and grouping them costs a dependent test per visit.
+// (Times beside smallEvents.)
+constexpr int kSmallBlock = 32, kSmallBatch = 8;
+template <int OP, bool TOF, bool COMP>
+__global__ void __launch_bounds__(kSmallBlock)
+    k_events_small(KParams P, Events E, Range R, const float* __restrict__ in,
+                   float* __restrict__ out, float globalScale, float denomThr,
+                   unsigned long long* err)
+{
+	const uint64_t k = static_cast<uint64_t>(blockIdx.x) * kSmallBlock + threadIdx.x;
+	const uint64_t e = R.start + k * R.stride;
+	float3 p1 = make_float3(0.f, 0.f, 0.f), p2 = p1, n1, n2;
+	bool ok = k < R.count;
+	int frame = 0;
+	if (ok)
+	{
+		frame = E.frame ? __ldg(E.frame + e) : 0;
+		ok = frame >= 0 && frame < P.g.nt && fetchEvent(P, E, e, p1, p2, n1, n2);
+		if (!ok)
+		{
+			if (frame >= 0)
+				atomicAdd(err, 1ULL);
+			if constexpr (OP == OP_FWD)
+				out[e] = 0.f;
+			if constexpr (OP == OP_EM)
+				if (E.model)
+					E.model[e] = 0.f;
+		}
+	}
+	const float tofv = TOF && ok ? __ldg(E.tof + e) : 0.f;
+	const int64_t fo = ok ? static_cast<int64_t>(frame) * P.g.nvox : 0;
+	float v = 0.f, m = 1.f, s = 1.f, a = 1.f;
+	if constexpr (OP == OP_BWD)
+	{
+		v = ok ? __ldg(in + e) : 0.f;
+	}
+	else
+	{
+		if (OP == OP_EM && ok)
+		{
+			m = E.meas ? __ldg(E.meas + e) : 1.0f;
+			s = E.sens ? __ldg(E.sens + e) : 1.0f;
+			a = E.att ? __ldg(E.att + e) : 1.0f;
+			if (m == 0.f || s == 0.f || a == 0.f)
+			{
+				if (E.model)
+					E.model[e] = 0.f;
+				ok = false;
+			}
+		}
+		const float* img = in + fo;
+		float ray = 0.f, comp = 0.f;
+		auto consume = [&](const int (&o)[kSmallBatch], const float (&w)[kSmallBatch])
+		{
+			float q[kSmallBatch];
+#pragma unroll
+			for (int j = 0; j < kSmallBatch; j++)
+				q[j] = o[j] >= 0 ? __ldg(img + o[j]) : 0.f;
+#pragma unroll
+			for (int j = 0; j < kSmallBatch; j++)
+			{
+				if (o[j] < 0)
+					continue;
+				if constexpr (COMP)
+				{
+					const float y = __fmaf_rn(w[j], q[j], -comp);
+					const float t = ray + y;
+					comp = (t - ray) - y;
+					ray = t;
+				}
+				else
+				{
+					ray += w[j] * q[j];
+				}
+			}
+		};
+		siddonWalkWarpBatched<TOF, COMP, kSmallBatch>(ok, P.g, p1, p2, P.tof, tofv, consume);
+		float u = 0.f + ray;
+		if constexpr (OP == OP_FWD)
+		{
+			if (ok)
+				out[e] = u;
+			return;
+		}
+		u *= s;
+		u *= a;
+		u *= globalScale;
+		if (ok && E.add)
+			u += __ldg(E.add + e);
+		if (ok && E.model)
+			E.model[e] = u;
+		ok = ok && fabsf(u) > denomThr;
+		u = m / u;
+		u *= s;
+		u *= a;
+		u *= globalScale;
+		v = u;
+	}
+	if (ok)
+		backwardEvent<K_SIDDON, TOF, COMP>(P, out + fo, v, p1, p2, n1, n2, tofv, k);
+}
+
 // Diagnostics: the (offset, weight) visits of each event's walk in walk
 // order, item k of the range at offs/wts[k * cap ...] (at most cap of them),
 // the number of visits in counts[k]; offsets within the event's frame.
@@ -2963,6 +3069,8 @@ struct yrtb_projector
 	uint64_t mrCapacity = 0;
 	// Launch configuration of the single-ray Siddon event kernels.
 	yrtb_launch_config launch{256, 1, 3, YRTB_ORDER_LOR, 1, 2};
+	// Set by the caller (yrtb_projector_set_launch) or the autotuner.
+	bool launchSet = false;
 	// Layout of the images of the list-mode projections (YRTB_LAYOUT_*).
 	int layout = YRTB_LAYOUT_ROW_MAJOR;
 	// Deterministic back projection: fixed-point image (nvox * nt) and bound.
@@ -3276,6 +3384,18 @@ inline int rayLanes(int numRays)
 	return l <= 8 ? l : 0;
 }
 
+// Most events of a launch that takes the small form.  128 x 128 x 64 voxels,
+// us small / default, TOF mirror and non-TOF compensated: forward 28 / 50 and
+// 30 / 53 at 16,000 events, 57 / 68 and 55 / 64 at 128,000, 104 / 101 and 101 /
+// 118 at 256,000; backward 21 / 31 and 23 / 36 at 16,000, 40 / 40 and 64 / 48 at
+// 64,000; EM pass 44 / 75 and 56 / 87 at 16,000, 70 / 83 and 99 / 98 at 64,000,
+// 119 / 128 and 159 / 149 at 128,000.
+template <int OP>
+constexpr uint64_t smallEvents()
+{
+	return OP == OP_FWD ? 131072 : OP == OP_EM ? 65536 : 32768;
+}
+
 // layout: the images' layout (YRTB_LAYOUT_*), -1 for the projector's.
 template <int OP>
 yrtb_status dispatchEvents(yrtb_projector* h, const yrtb_events* ev,
@@ -3312,7 +3432,16 @@ yrtb_status dispatchEvents(yrtb_projector* h, const yrtb_events* ev,
 		{
 			if (!(kScatter && h->det))
 			{
-				if (tiled)
+				// The small form replaces the default launch shape only: one
+				// that was set is kept.
+				if (!tiled && R.count <= smallEvents<OP>() && h->launch.threads_per_lor == 1 &&
+				    !h->launchSet)
+				{
+					k_events_small<OP, T, C>
+					    <<<static_cast<unsigned>((R.count + kSmallBlock - 1) / kSmallBlock),
+					       kSmallBlock, 0, st>>>(h->P, E, R, in, out, gs, thr, h->d_err);
+				}
+				else if (tiled)
 				{
 					if (h->launch.block == 128)
 						launchTuned<OP, K, T, C, 128, true>(h, E, R, in, out, gs, thr, st, F);
@@ -4075,6 +4204,7 @@ yrtb_status yrtb_projector_set_launch(yrtb_projector* h,
 	if (c->vector_groups < 0 || c->vector_groups > 15)
 		return fail(YRTB_ERR_ARGUMENT, "vector_groups must be in 0..15");
 	h->launch = *c;
+	h->launchSet = true;
 	return YRTB_OK;
 }
 
@@ -5715,6 +5845,7 @@ yrtb_status yrtb_autotune(yrtb_projector* h, const float* d_image,
 	cudaMemsetAsync(em, 0, J * 4, st);
 
 	const yrtb_launch_config saved = h->launch;
+	h->launchSet = true;  // the configurations are timed as they are
 	cudaEvent_t e0 = nullptr, e1 = nullptr;
 	cudaEventCreate(&e0);
 	cudaEventCreate(&e1);
