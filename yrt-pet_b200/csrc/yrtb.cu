@@ -2702,6 +2702,7 @@ constexpr int kLrMaxRank = 32;
 constexpr int kLrTile = 128;      // voxels per shared-memory tile (H contraction)
 constexpr int kLrPairs = 8;       // rank x frames <= 8 x 256
 constexpr int kLrBlock = 256;
+constexpr int kLrBlocksPerSM = 3;  // one block loads its tile while others add
 
 // X[t][j] = sum_l W[l][j] * H[l][t], l ascending, rounded products and sums
 // (the CPU updater's forwardUpdate order).
@@ -2831,8 +2832,10 @@ k_lr_contract_w4(const float4* __restrict__ E, const float* __restrict__ H, int 
 // and 8 conversions to FP64 (the slow unit) serve 16 multiply-adds.  With one
 // pair per thread they served one, most of the 256 threads had no pair (120 of
 // rank 6, 20 frames) and every product was converted; a reconstruction of rank 6,
-// 20 frames, 4 subsets of 1M voxels, 2M events took 3.21 ms, and takes 2.87.
-__global__ void __launch_bounds__(kLrBlock)
+// 20 frames, 4 subsets of 1M voxels, 2M events took 3.21 ms, 2.87 with this, and
+// 2.26 with 3 blocks per SM, a warp per pair in k_lr_finish and the EM pass's
+// batched walk.
+__global__ void __launch_bounds__(kLrBlock, kLrBlocksPerSM)
 k_lr_contract_h(const float* __restrict__ W, const float* __restrict__ E, int R, int T,
                 uint64_t J, double* __restrict__ partial)
 {
@@ -2913,17 +2916,22 @@ k_lr_contract_h(const float* __restrict__ W, const float* __restrict__ E, int R,
 	}
 }
 
-// out[k] = sum over blocks b (ascending) of partial[b][k].
+// out[k] = sum over blocks b of partial[b][k], one warp per pair: lane l adds
+// the blocks l, l + 32, ... in order, then the lanes are added as a tree.  (One
+// thread per pair waited for 296 loads in turn: 46 us.)
 __global__ void k_lr_finish(const double* __restrict__ partial, int blocks, int P,
                             double* __restrict__ out)
 {
-	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P; k += gridDim.x * blockDim.x)
-	{
-		double s = 0.0;
-		for (int b = 0; b < blocks; b++)
-			s += partial[static_cast<uint64_t>(b) * P + k];
+	const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+	if (k >= P)
+		return;  // whole warps
+	double s = 0.0;
+	for (int b = lane; b < blocks; b += 32)
+		s += partial[static_cast<uint64_t>(b) * P + k];
+	for (int o = 16; o > 0; o >>= 1)
+		s += __shfl_down_sync(0xffffffffu, s, o);
+	if (lane == 0)
 		out[k] = s;
-	}
 }
 
 // H[r][t] *= float(Hn[r][t]) * (1 / max(cH[r], eps))  (LREM::applyHUpdate,
@@ -5273,11 +5281,11 @@ yrtb_status yrtb_lr_contract_h(const float* d_W, const float* d_E, int R, int T,
 		                               cudaFuncAttributeMaxDynamicSharedMemorySize,
 		                               static_cast<int>(smem)));
 	const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>(
-	    (J + kLrTile - 1) / kLrTile, static_cast<uint64_t>(gridFor(1 << 30, 2))));
+	    (J + kLrTile - 1) / kLrTile, static_cast<uint64_t>(gridFor(1 << 30, kLrBlocksPerSM))));
 	double* partial = nullptr;
 	YRTB_CUDA(poolAlloc(&partial, static_cast<size_t>(blocks) * P * sizeof(double), st));
 	k_lr_contract_h<<<blocks, kLrBlock, smem, st>>>(d_W, d_E, R, T, J, partial);
-	k_lr_finish<<<(P + kBlock - 1) / kBlock, kBlock, 0, st>>>(partial, blocks, P, d_Hn);
+	k_lr_finish<<<(32 * P + kBlock - 1) / kBlock, kBlock, 0, st>>>(partial, blocks, P, d_Hn);
 	YRTB_CUDA(cudaFreeAsync(partial, st));
 	YRTB_LAUNCHED();
 	return YRTB_OK;
