@@ -1066,20 +1066,27 @@ __global__ void __launch_bounds__(BLOCK, ((KIND == K_SIDDON && COMP) ||
 	}
 }
 
-// Small launches of the single-ray Siddon operations: too few rays to hide the
-// latency of their image reads, so a walk records 8 crossings, issues their
-// reads together and adds them in walk order (the same sums as k_events), and
-// blocks of one warp spread over all SMs.  Reductions are sent per voxel: the
-// L2 has room, and grouping them costs a dependent test per visit.
-// (Times beside smallEvents.)
-constexpr int kSmallBlock = 32, kSmallBatch = 8;
-template <int OP, bool TOF, bool COMP>
-__global__ void __launch_bounds__(kSmallBlock)
-    k_events_small(KParams P, Events E, Range R, const float* __restrict__ in,
+// The single-ray Siddon operations with a batched forward walk: the lanes of a
+// warp walk in lock step, record 8 crossings, issue their reads together and
+// add them in walk order (the same sums as k_events).  Walked one crossing at a
+// time a ray waits for each of its reads in turn, which few rays cannot hide
+// and a full machine hides only in part: 3M TOF events in file order, log-
+// likelihood and gradient 1724 -> 1481 us; OSEM of 1M events without TOF 2.22 ->
+// 2.01 ms, of 20M TOF events (L2-bound) 35.6 -> 34.5 ms.  4 crossings measured
+// 1491 us, 2.01 and 34.5 ms.
+// BLOCK kSmallBlock: small launches, in blocks of one warp that spread over all
+// SMs, with reductions per voxel: the L2 has room, and grouping them costs a
+// dependent test per visit (times beside smallEvents).  Other blocks: the
+// launch shape's, at k_events' threads per SM.
+constexpr int kSmallBlock = 32, kWalkBatch = 8;
+// RED: the back projection's reductions (backwardEvent's VEC).
+template <int OP, bool TOF, bool COMP, int BLOCK = kSmallBlock, int RED = 0>
+__global__ void __launch_bounds__(BLOCK, BLOCK == kSmallBlock ? 1 : (COMP ? 1024 : 768) / BLOCK)
+    k_events_batch(KParams P, Events E, Range R, const float* __restrict__ in,
                    float* __restrict__ out, float globalScale, float denomThr,
                    unsigned long long* err)
 {
-	const uint64_t k = static_cast<uint64_t>(blockIdx.x) * kSmallBlock + threadIdx.x;
+	const uint64_t k = static_cast<uint64_t>(blockIdx.x) * BLOCK + threadIdx.x;
 	const uint64_t e = R.start + k * R.stride;
 	float3 p1 = make_float3(0.f, 0.f, 0.f), p2 = p1, n1, n2;
 	bool ok = k < R.count;
@@ -1122,14 +1129,14 @@ __global__ void __launch_bounds__(kSmallBlock)
 		}
 		const float* img = in + fo;
 		float ray = 0.f, comp = 0.f;
-		auto consume = [&](const int (&o)[kSmallBatch], const float (&w)[kSmallBatch])
+		auto consume = [&](const int (&o)[kWalkBatch], const float (&w)[kWalkBatch])
 		{
-			float q[kSmallBatch];
+			float q[kWalkBatch];
 #pragma unroll
-			for (int j = 0; j < kSmallBatch; j++)
+			for (int j = 0; j < kWalkBatch; j++)
 				q[j] = o[j] >= 0 ? __ldg(img + o[j]) : 0.f;
 #pragma unroll
-			for (int j = 0; j < kSmallBatch; j++)
+			for (int j = 0; j < kWalkBatch; j++)
 			{
 				if (o[j] < 0)
 					continue;
@@ -1146,7 +1153,7 @@ __global__ void __launch_bounds__(kSmallBlock)
 				}
 			}
 		};
-		siddonWalkWarpBatched<TOF, COMP, kSmallBatch>(ok, P.g, p1, p2, P.tof, tofv, consume);
+		siddonWalkWarpBatched<TOF, COMP, kWalkBatch>(ok, P.g, p1, p2, P.tof, tofv, consume);
 		float u = 0.f + ray;
 		if constexpr (OP == OP_FWD)
 		{
@@ -1169,7 +1176,7 @@ __global__ void __launch_bounds__(kSmallBlock)
 		v = u;
 	}
 	if (ok)
-		backwardEvent<K_SIDDON, TOF, COMP>(P, out + fo, v, p1, p2, n1, n2, tofv, k);
+		backwardEvent<K_SIDDON, TOF, COMP, false, RED>(P, out + fo, v, p1, p2, n1, n2, tofv, k);
 }
 
 // Diagnostics: the (offset, weight) visits of each event's walk in walk
@@ -3309,6 +3316,28 @@ void launchTuned(const yrtb_projector* h, const Events& E, Range R,
 		constexpr int TPL = decltype(tplc)::value;
 		const uint64_t threads = R.count * TPL;
 		const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, (threads + B - 1) / B));
+		constexpr bool kBatched = OP == OP_EM && K == K_SIDDON && TPL == 1 && !TILE;
+		if constexpr (kBatched)
+		{
+			// Without float4 gathers or staged reductions, the form whose
+			// forward walk is batched.
+			const int groups = aligned ? h->launch.vector_groups & (quads ? 15 : 14) : 0;
+			if (!(groups & 5))
+			{
+				auto batch = [&](auto red)
+				{
+					k_events_batch<OP, T, C, B, decltype(red)::value>
+					    <<<grid, B, 0, st>>>(h->P, E, R, in, out, gs, thr, h->d_err);
+				};
+				if (groups & 2)
+					batch(std::integral_constant<int, 1>{});
+				else if (groups & 8)
+					batch(std::integral_constant<int, 3>{});
+				else
+					batch(std::integral_constant<int, 0>{});
+				return;
+			}
+		}
 		if constexpr (TPL == 1 || K == K_SIDDON_MR)
 		{
 			// Bit 0: float4 gathers (forward); bit 1: float4 reductions summed
@@ -3330,7 +3359,7 @@ void launchTuned(const yrtb_projector* h, const Events& E, Range R,
 				auto vlaunch = [&](auto vc)
 				{
 					constexpr int V = decltype(vc)::value;
-					if constexpr ((V & kUse) == V)
+					if constexpr ((V & kUse) == V && (!kBatched || (V & 5)))
 						k_events<OP, K, T, C, false, B, TPL, V, TILE><<<grid, B, 0, st>>>(
 						    h->P, E, R, in, out, gs, thr, h->d_err, F);
 				};
@@ -3347,8 +3376,9 @@ void launchTuned(const yrtb_projector* h, const Events& E, Range R,
 				return;
 			}
 		}
-		k_events<OP, K, T, C, false, B, TPL, 0, TILE><<<grid, B, 0, st>>>(h->P, E, R, in, out, gs,
-		                                                        thr, h->d_err, F);
+		if constexpr (!kBatched)
+			k_events<OP, K, T, C, false, B, TPL, 0, TILE><<<grid, B, 0, st>>>(
+			    h->P, E, R, in, out, gs, thr, h->d_err, F);
 	};
 	int tpl = h->launch.threads_per_lor;
 	if constexpr (K == K_SIDDON_MR)
@@ -3398,10 +3428,14 @@ inline int rayLanes(int numRays)
 // 118 at 256,000; backward 21 / 31 and 23 / 36 at 16,000, 40 / 40 and 64 / 48 at
 // 64,000; EM pass 44 / 75 and 56 / 87 at 16,000, 70 / 83 and 99 / 98 at 64,000,
 // 119 / 128 and 159 / 149 at 128,000.
-template <int OP>
+// A forward projection takes it at any size but in mirror arithmetic without TOF
+// (3M events, file order / sorted, us: compensated TOF 986 / 560 -> 658 / 408,
+// mirror TOF 1346 / 720 -> 1118 / 667, compensated 1171 / 787 -> 996 / 740, but
+// mirror 1205 / 835 -> 1220 / 921).
+template <int OP, bool TOF, bool COMP>
 constexpr uint64_t smallEvents()
 {
-	return OP == OP_FWD ? 131072 : OP == OP_EM ? 65536 : 32768;
+	return OP == OP_FWD ? ((TOF || COMP) ? ~uint64_t(0) : 524288) : OP == OP_EM ? 65536 : 32768;
 }
 
 // layout: the images' layout (YRTB_LAYOUT_*), -1 for the projector's.
@@ -3442,10 +3476,11 @@ yrtb_status dispatchEvents(yrtb_projector* h, const yrtb_events* ev,
 			{
 				// The small form replaces the default launch shape only: one
 				// that was set is kept.
-				if (!tiled && R.count <= smallEvents<OP>() && h->launch.threads_per_lor == 1 &&
-				    !h->launchSet)
+				if (!tiled && R.count <= smallEvents<OP, T, C>() &&
+				    h->launch.threads_per_lor == 1 &&
+				    (OP == OP_FWD ? !(h->launch.vector_groups & 1) : !h->launchSet))
 				{
-					k_events_small<OP, T, C>
+					k_events_batch<OP, T, C>
 					    <<<static_cast<unsigned>((R.count + kSmallBlock - 1) / kSmallBlock),
 					       kSmallBlock, 0, st>>>(h->P, E, R, in, out, gs, thr, h->d_err);
 				}
