@@ -198,3 +198,133 @@ def test_osem_deterministic_graph_and_plain_bit_identical():
         outs.append(osem.reconstruct().cpu().numpy())
     assert np.array_equal(outs[0].view(np.uint32), outs[1].view(np.uint32))
     assert np.array_equal(outs[1].view(np.uint32), outs[2].view(np.uint32))
+
+
+def exact_back(p, ev, v, rays, ip):
+    """(FP64 sum of the walks' FP32 weights times the values, largest |v w|
+    of the value before its share per ray)."""
+    offs, wts, cnt = p.trace_walks(ev, cap=512)
+    assert int(cnt.max()) <= offs.shape[1]
+    on = torch.arange(offs.shape[1], device="cuda")[None] < cnt[:, None]
+    c = (v / torch.full_like(v, rays)).double()[:, None] * wts.double()
+    c = torch.where(on, c, 0.0)
+    img = torch.zeros(ip.numVoxels, dtype=torch.float64, device="cuda")
+    img.index_add_(0, offs[on].long(), c[on])
+    return img.reshape(ip.shape), rays * float(c.abs().max())
+
+
+def assert_exact(img, want, largest, n, rays):
+    # n roundings to units of 2^-61 of the power of two above n M, and one of
+    # the sum to FP32.
+    unit = 2.0 ** -60 * n * largest
+    err = (img.double() - want).abs()
+    assert bool((err <= rays * n * unit + 2.0 ** -23 * want.abs()).all())
+
+
+def reciprocal(y, miss):
+    # (The sums of a TOF tail are no normal numbers: 0 for those.)
+    v = torch.where(y > 1e-30, 1.0 / y, 0.0)
+    return torch.where(y == 0, torch.tensor(miss, device="cuda"), v)
+
+
+# 1 / (A x), as a Poisson gradient or MLEM back-projects it: largest where a ray
+# clips a corner or the TOF window's tail, and 1 / eps on the rays that miss the
+# grid, which reach no voxel and must not coarsen the others' sums.
+@pytest.mark.parametrize("projector,tof,rays,prec", CASES)
+@pytest.mark.parametrize("miss", [1e12, 1e38])
+def test_backward_of_reciprocal_values_is_exact(projector, tof, rays, prec, miss):
+    # Short along z: oblique rays clip the grid's edges.
+    sc, ip, p = make(projector, tof, rays, prec, ip_args=(32, 32, 16, 128, 128, 30))
+    d1, d2 = random_events(20000, 40)
+    rng = np.random.default_rng(41)
+    tv = rng.normal(0, 500, len(d1)).astype(np.float32) if tof else None
+    ev = yrt.DeviceEvents.from_arrays(d1, d2, tof=tv)
+    y = p.forward(torch.ones(ip.shape, device="cuda"), ev)
+    assert int((y == 0).sum()) > 100 and float(y[y > 0].min()) < 0.1 * float(y.max())
+    v = reciprocal(y, miss)
+    want, largest = exact_back(p, ev, v, rays, ip)
+    assert_exact(p.backward(v, ev), want, largest, len(d1), rays)
+
+
+HISTO_SC = (40, 4, 4, 10, 100, 32, 6, 1, 4, 3, 1)
+HISTO_IP = (21, 18, 10, 60.0, 50.0, 20.0)
+
+
+def histo_case(projector, rays, prec, subsets, subset):
+    sc = yrt.Scanner("t", *HISTO_SC)
+    ip = yrt.ImageParams(*HISTO_IP)
+    pp = yrt.ProjectorParams(sc)
+    pp.setProjector(projector)
+    pp.numRays = rays
+    pp.precision = prec
+    pp.deterministic = True
+    p = yrt.DeviceProjector(sc, ip, pp)
+    h = yrt.Histogram3D(sc)
+    bins = h.getBinIter(subsets, subset).indices()
+    ev = yrt.DeviceEvents.from_arrays(*yrt.histo3d_detpairs(sc, bins))
+    idx = torch.from_numpy(bins.astype(np.int64)).cuda()
+    y = p.forward(torch.ones(ip.shape, device="cuda"), ev)
+    assert int((y == 0).sum()) > 100
+    return sc, ip, p, h, ev, idx, y
+
+
+@pytest.mark.parametrize("projector,rays", [("S", 1), ("S", 3), ("DD", 1)])
+@pytest.mark.parametrize("prec", [L.YRTB_MIRROR, L.YRTB_COMPENSATED])
+@pytest.mark.parametrize("miss", [1e12, 1e38])
+def test_histogram_back_projection_of_reciprocal_values_is_exact(projector, rays, prec, miss):
+    sc, ip, p, h, ev, idx, y = histo_case(projector, rays, prec, 2, 1)
+    v = reciprocal(y, miss)
+    full = torch.full((h.histoSize,), 3.0, device="cuda")
+    full[idx] = v
+    img = p.backward_histo3d(full, torch.zeros(ip.shape, device="cuda"), 2, 1)
+    want, largest = exact_back(p, ev, v, rays, ip)
+    assert_exact(img, want, largest, len(v), rays)
+    sens = torch.zeros(ip.shape, device="cuda")
+    p.sensitivity_histo3d(sens, 2, 1, sens_histo=full)
+    if rays > 1 and prec == L.YRTB_COMPENSATED:
+        # Sensitivity images of several rays are projected in mirror
+        # arithmetic whatever the precision.
+        p = histo_case(projector, rays, L.YRTB_MIRROR, 2, 1)[2]
+        want, largest = exact_back(p, ev, v, rays, ip)
+    assert_exact(sens, want, largest, len(v), rays)
+
+
+# A value that is not finite makes the whole image NaN, also on a ray that
+# misses the grid (|v| max|w| is inf * 0).
+@pytest.mark.parametrize("projector,rays", [("S", 1), ("S", 3), ("DD", 1)])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_values_not_finite_on_missing_rays_poison_the_image(projector, rays, bad):
+    sc, ip, p, h, ev, idx, y = histo_case(projector, rays, L.YRTB_COMPENSATED, 1, 0)
+    # (A bin whose two crystals coincide has no ray.)
+    pair = ev.d1 != ev.d2
+    where = int(torch.nonzero((y == 0) & pair)[0])
+    v = torch.ones_like(y)
+    v[where] = bad
+    assert p.backward(v, ev).isnan().all()
+    full = torch.ones(h.histoSize, device="cuda")
+    full[idx] = v
+    zeros = lambda: torch.zeros(ip.shape, device="cuda")
+    assert p.backward_histo3d(full, zeros()).isnan().all()
+    assert p.sensitivity_histo3d(zeros(), sens_histo=full).isnan().all()
+    assert p.sensitivity_histo3d(zeros(), acf_histo=full).isnan().all()
+    x = torch.ones(ip.shape, device="cuda")
+    add = torch.ones_like(full)
+    assert p.em_step_histo3d(x, zeros(), full, 1, 0, additive_histo=add).isnan().all()
+    # Without an additive term such a bin's model is 0: below the threshold.
+    assert p.em_step_histo3d(x, zeros(), full, 1, 0).isfinite().all()
+    # The product of two crystals' factors overflows on one pair only.
+    eff = torch.ones(sc.getNumDets(), device="cuda")
+    eff[ev.d1[where].long()] = 1e30
+    eff[ev.d2[where].long()] = 1e30
+    assert p.sensitivity_histo3d(zeros(), crystal_eff=eff).isnan().all()
+    # An attenuation image that reaches past the grid, NaN in one voxel that
+    # only rays that miss the grid cross.
+    mp = yrt.ImageParams(42, 36, 20, 180.0, 150.0, 36.0)
+    offs, _, cnt = yrt.DeviceProjector(sc, mp, yrt.ProjectorParams(sc)).trace_walks(ev, cap=128)
+    on = torch.arange(128, device="cuda")[None] < cnt[:, None]
+    seen = [torch.bincount(offs[on & rows[:, None]].long(), minlength=mp.numVoxels) > 0
+            for rows in (y == 0, y > 0)]
+    mu = torch.zeros(mp.shape, device="cuda")
+    assert p.sensitivity_histo3d(zeros(), mu=mu, mu_params=mp).isfinite().all()
+    mu.view(-1)[int(torch.nonzero(seen[0] & ~seen[1])[0])] = np.nan
+    assert p.sensitivity_histo3d(zeros(), mu=mu, mu_params=mp).isnan().all()

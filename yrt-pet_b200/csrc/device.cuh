@@ -618,6 +618,20 @@ struct SiddonWalker
 			rz--;
 	}
 
+	// Upper bound of the walk's segments (after a successful begin): the first
+	// one, and for the others, on each axis, the distance to its next plane or
+	// between two of its planes, whichever is larger.  The margins cover the
+	// rounding of crossings (a few units of 2^-24 of the ray) and of planes
+	// (relative 2^-24 per voxel of the axis).
+	__device__ __forceinline__ float segmentBound() const
+	{
+		const float x = fmaxf(ax_next - a_next, fabsf(fdx * inv_x));
+		const float y = fmaxf(ay_next - a_next, fabsf(fdy * inv_y));
+		const float z = fmaxf(az_next - a_next, fabsf(fdz * inv_z));
+		const float a = fmaxf(a_next - a_cur, fminf(fminf(x, y), z));
+		return d_norm * (a * 1.002f + 1e-6f);
+	}
+
 	template <typename Visit>
 	__device__ __forceinline__ void emitFirst(Visit& visit)
 	{
@@ -700,6 +714,28 @@ __device__ __forceinline__ void siddonWalkWarp(bool alive, const Geom& g,
 		if (alive)
 			alive = w.next(visit);
 	}
+}
+
+// Largest |weight| of each lane's ray, in lock step and without image reads; 0
+// for rays whose bound needed(bound) says is of no interest.
+template <bool COMP, typename Needed>
+__device__ __forceinline__ float siddonMaxWeightWarp(bool alive, const Geom& g, const float3 p1,
+                                                     const float3 p2, const TofP& tp,
+                                                     Needed& needed)
+{
+	SiddonWalker<false, COMP> w;
+	if (alive)
+		alive = w.begin(g, p1, p2, tp, 0.f, 0.f, 1.f, 0, 1) && needed(w.segmentBound());
+	float mw = 0.f;
+	auto visit = [&](int, float wt) { mw = fmaxf(mw, fabsf(wt)); };
+	if (alive)
+		w.emitFirst(visit);
+	while (__any_sync(0xffffffffu, alive))
+	{
+		if (alive)
+			alive = w.next(visit);
+	}
+	return mw;
 }
 
 // siddonWalkWarp in batches of B crossings: each round every lane takes up

@@ -635,8 +635,10 @@ __device__ __forceinline__ float maxWeightEvent(const KParams& P, float3 p1,
 // ------------------------------------------- deterministic back projection --
 // Two passes.  Pass 1 reduces M = max over events of |v_e| * max_k |w_ek|
 // (v_e the value back-projected along event e, w_ek its voxel weights; for
-// multi-ray, the rays of one event add at most |v_e| max|w| to a voxel).  Any
-// voxel then receives at most n * M in magnitude from the n events of the
+// multi-ray, the rays of one event add at most |v_e| max|w| to a voxel).  The
+// weights are those of the walk itself: values like 1 / (A x) are largest where
+// the weights are smallest, or where a ray misses the grid and has none, and a
+// bound from the voxel's diagonal left such images without a bit.  Any voxel then receives at most n * M in magnitude from the n events of the
 // call.  Pass 2 scatters round(v_e * w_ek * 2^s) into 64-bit integers with
 // 2^s the largest power of two for which n * M * 2^s <= 2^61, so the integer
 // sums cannot overflow (the roundings add at most numRays * n / 2 < 2^62).
@@ -648,18 +650,6 @@ struct Fixed
 	const unsigned* maxBits;  // M as float bits (pass 1 result)
 	uint64_t n;               // events (bins) of the call
 };
-
-// Siddon rays: |w| is a segment's length (times at most the TOF peak), and a
-// segment lies between two planes of each axis one voxel apart, so it is not
-// longer than the voxel's diagonal; a first plane misplaced by one in FP32
-// doubles that.  Twice as much again as margin: M may be too large (2 bits of
-// the 61 per factor of 4), not too small.  Knowing it, the bound of a value
-// given per event needs no walk.
-__host__ __device__ inline float siddonWeightBound(const KParams& P, bool tof)
-{
-	const float d = sqrtf(P.g.vx * P.g.vx + P.g.vy * P.g.vy + P.g.vz * P.g.vz);
-	return 4.f * d * (tof ? P.tof.norm : 1.f);
-}
 
 // Exponent k with n * M < 2^k; 0x7fffffff when M is zero or not finite.
 __device__ __forceinline__ int fixedExponent(unsigned maxBits, uint64_t n)
@@ -677,6 +667,17 @@ __device__ __forceinline__ double fixedScale(const Fixed& F)
 {
 	const int k = fixedExponent(*F.maxBits, F.n);
 	return k == 0x7fffffff ? 0.0 : ldexp(1.0, 61 - k);
+}
+
+// Pass 1 in progress: only a product |v| max|w| of at least this (0: any) can
+// still change the exponent, which is all that pass 2 takes from M.  Once the
+// first blocks have set it, few rays' bounds reach it: an attenuated
+// sensitivity image of 8.3M bins takes 7.27 ms with every ray walked for its
+// weights, 6.13 ms with those that can matter.
+__device__ __forceinline__ double fixedHeadroom(const unsigned* maxBits, uint64_t n)
+{
+	const int k = fixedExponent(__ldcg(maxBits), n);
+	return k == 0x7fffffff ? 0.0 : ldexp(1.0, k) / static_cast<double>(n);
 }
 
 // Warp max of a non-negative float (as bits) folded into *out by lane 0.  All
@@ -1242,9 +1243,7 @@ __global__ void __launch_bounds__(kBlock, KIND == K_SIDDON ? 4 : 1)
 			if constexpr (!EM)
 			{
 				const float v = __ldg(in + e);
-				if constexpr (KIND == K_SIDDON || KIND == K_SIDDON_MR)
-					b = fabsf(v) * siddonWeightBound(P, TOF);
-				else if (v != 0.f)
+				if (v != 0.f)
 					b = fabsf(v) * maxWeightEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2,
 					                                                tofv, k);
 			}
@@ -1595,6 +1594,33 @@ struct HistoArgs
 	float* stored;
 };
 
+// LOR sensitivity of a bin: a histogram value, or the product of the two
+// crystals' factors (the same FP32 product a histogram of them holds).
+__device__ __forceinline__ float histoSens(const HistoArgs& A, uint64_t bin, uint32_t d1,
+                                           uint32_t d2)
+{
+	return A.sensH ? __ldg(A.sensH + bin)
+	               : (A.crystalEff ? __ldg(A.crystalEff + d1) * __ldg(A.crystalEff + d2) : 1.0f);
+}
+
+// EM ratio of a bin from its forward projection u; ok (the bin takes part)
+// becomes false where the model is not above the threshold.
+__device__ __forceinline__ float histoRatio(const HistoArgs& A, uint64_t bin, float m, float u,
+                                            float s, float a, bool& ok)
+{
+	u *= s;
+	u *= a;
+	u *= A.globalScale;
+	if (A.addH && ok)
+		u += __ldg(A.addH + bin);
+	ok = ok && fabsf(u) > A.denomThr;
+	u = m / u;
+	u *= s;
+	u *= a;
+	u *= A.globalScale;
+	return u;
+}
+
 // Blocks per SM of the compensated DD + PSF histogram EM kernel (several
 // threads per bin).
 constexpr int kDDPsfBlocksPerSM = 3;
@@ -1646,8 +1672,6 @@ __device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, cons
 			n2 = make_float3(ob.x, ob.y, ob.z);
 		}
 	}
-	// LOR sensitivity: a histogram value, or the product of the two crystals'
-	// factors (the same FP32 product a histogram of them holds).
 	float s = 1.f, a = 1.f, v = 0.f;
 	const bool ready = HOP == HOP_SENS && MODE == H_FIX && A.stored != nullptr;
 	if (HOP == HOP_BWD)
@@ -1661,9 +1685,7 @@ __device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, cons
 	else if (HOP != HOP_FWD)
 	{
 		if (ok)
-			s = A.sensH ? __ldg(A.sensH + bin)
-			            : (A.crystalEff ? __ldg(A.crystalEff + d1) * __ldg(A.crystalEff + d2)
-			                            : 1.0f);
+			s = histoSens(A, bin, d1, d2);
 		if (A.acfH)
 		{
 			a = ok ? __ldg(A.acfH + bin) : 1.f;
@@ -1720,17 +1742,7 @@ __device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, cons
 				A.vals[bin] = u;
 			return;
 		}
-		u *= s;
-		u *= a;
-		u *= A.globalScale;
-		if (A.addH && ok)
-			u += __ldg(A.addH + bin);
-		ok = ok && fabsf(u) > A.denomThr;
-		u = m / u;
-		u *= s;
-		u *= a;
-		u *= A.globalScale;
-		v = u;
+		v = histoRatio(A, bin, m, u, s, a, ok);
 		if constexpr (MODE == H_BOUND)
 			bound = ok ? fabsf(v) * mw : 0.f;
 	}
@@ -1738,15 +1750,20 @@ __device__ __forceinline__ void histoItem(const KParams& P, const H3Dev& H, cons
 	{
 		if (A.stored && exists)
 			A.stored[t] = v;
-		if (ok)
+		const bool walk = ok && v != 0.f;
+		float mw = 0.f;
+		if constexpr (WARP)
 		{
-			if constexpr (KIND == K_SIDDON || KIND == K_SIDDON_MR)
-				bound = fabsf(v) * siddonWeightBound(P, false);
-			else
-				bound = fabsf(v) *
-				        (v != 0.f ? maxWeightEvent<KIND, false, COMP>(P, p1, p2, n1, n2, 0.f, k)
-				                  : 0.f);
+			const double enough = fixedHeadroom(A.maxBits, A.F.n);
+			auto needed = [&](float most)
+			{ return !(static_cast<double>(fabsf(v)) * static_cast<double>(most) < enough); };
+			mw = siddonMaxWeightWarp<COMP>(walk, P.g, p1, p2, P.tof, needed);
 		}
+		else if (walk)
+		{
+			mw = maxWeightEvent<KIND, false, COMP>(P, p1, p2, n1, n2, 0.f, k);
+		}
+		bound = walk ? fabsf(v) * mw : 0.f;
 	}
 	if constexpr (MODE == H_BOUND)
 	{
@@ -1779,6 +1796,36 @@ __global__ void __launch_bounds__(kBlock, (KIND == K_DD_PSF && TPL > 1) ? kDDPsf
 	                                             static_cast<int>(gt % TPL));
 }
 
+// Whether the value of a bin whose ray misses the grid is known to be finite
+// without a walk.
+template <int HOP>
+__device__ __forceinline__ bool idleFinite(const KParams& P, const HistoArgs& A, uint64_t bin,
+                                           uint32_t d1, uint32_t d2)
+{
+	if constexpr (HOP == HOP_BWD)
+	{
+		return isfinite(__ldg(A.vals + bin));
+	}
+	else
+	{
+		if (!A.acfH && A.muImg)
+		{
+			const float4 pa = __ldg(P.scan.pos + d1), pb = __ldg(P.scan.pos + d2);
+			const float3 off = make_float3(A.mu.offx, A.mu.offy, A.mu.offz);
+			if (crossesGrid(A.mu, f3sub(make_float3(pa.x, pa.y, pa.z), off),
+			                f3sub(make_float3(pb.x, pb.y, pb.z), off)))
+				return false;
+		}
+		const float s = histoSens(A, bin, d1, d2), a = A.acfH ? __ldg(A.acfH + bin) : 1.f;
+		if constexpr (HOP == HOP_SENS)
+			return isfinite(a * s);
+		const float m = __ldg(A.meas + bin);
+		bool ok = m != 0.f;
+		const float v = histoRatio(A, bin, m, 0.f, s, a, ok);
+		return !ok || isfinite(v);
+	}
+}
+
 // Single-ray Siddon: a block takes kSiddonTile items, lists those whose ray
 // crosses the grid, in order, and walks the list.  On 256 x 16 crystals of 300
 // mm radius and a 256 mm field only 27 % of the bins cross it, in runs of 35
@@ -1786,8 +1833,8 @@ __global__ void __launch_bounds__(kBlock, (KIND == K_DD_PSF && TPL > 1) ? kDDPsf
 // working warps without a ray.  384 items give 128 threads about one list's
 // worth there and about two where most bins cross.  693,000 bins, 128 x 128 x
 // 64 voxels, lock step without and with the list: forward 258 -> 127 us, back
-// 209 -> 175 us; the attenuated sensitivity image's first pass 1.99 -> 1.15 ms,
-// its second 1.74 -> 1.95 (64-bit reductions at the L2's limit).
+// 209 -> 175 us; the attenuated sensitivity image's first pass 1.99 -> 1.15 ms
+// (without the walk for its weights), its second 1.74 -> 1.95 (64-bit reductions at the L2's limit).
 constexpr int kSiddonBlock = 128, kSiddonTile = 3 * kSiddonBlock;
 template <int HOP, int MODE, bool COMP>
 __global__ void __launch_bounds__(kSiddonBlock, 8)
@@ -1798,7 +1845,6 @@ __global__ void __launch_bounds__(kSiddonBlock, 8)
 	const uint64_t first = static_cast<uint64_t>(blockIdx.x) * kSiddonTile;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	int n = 0;
-	float idle = 0.f;  // H_BOUND: NaN if a bin without a walk has no finite value
 #pragma unroll
 	for (int i = 0; i < kSiddonTile; i += kSiddonBlock)
 	{
@@ -1820,23 +1866,12 @@ __global__ void __launch_bounds__(kSiddonBlock, 8)
 			}
 			if (HOP == HOP_FWD && !in)
 				A.vals[bin] = 0.f;
-			if (MODE == H_BOUND && pair && !in)
+			if constexpr (MODE == H_BOUND)
 			{
-				if (HOP == HOP_BWD)
-					idle += 0.f * __ldg(A.vals + bin);
-				if (HOP == HOP_SENS && A.sensH)
-					idle += 0.f * __ldg(A.sensH + bin);
-				if (HOP == HOP_SENS && A.acfH)
-					idle += 0.f * __ldg(A.acfH + bin);
-				if (HOP == HOP_EM && A.addH)
-				{
-					// The ratio of a bin whose model is its additive term.
-					const float m = __ldg(A.meas + bin), u = __ldg(A.addH + bin);
-					const float c = (A.sensH ? __ldg(A.sensH + bin) : 1.f) *
-					                (A.acfH ? __ldg(A.acfH + bin) : 1.f) * A.globalScale;
-					if (m != 0.f && fabsf(u) > A.denomThr)
-						idle += 0.f * (m / u * c);
-				}
+				// A bin whose value is not finite, or may not be once its
+				// attenuation is walked, is listed all the same: |v| * 0 = NaN.
+				if (pair && !in)
+					in = !idleFinite<HOP>(P, A, bin, d1, d2);
 			}
 		}
 		const unsigned ballot = __ballot_sync(0xffffffffu, in);
@@ -1854,8 +1889,6 @@ __global__ void __launch_bounds__(kSiddonBlock, 8)
 			list[at] = static_cast<uint16_t>(i + threadIdx.x);
 		__syncthreads();
 	}
-	if (MODE == H_BOUND && idle != idle)
-		atomicMax(A.maxBits, 0x7fffffffu);
 	for (int j = warp * 32; j < n; j += kSiddonBlock)  // uniform over a warp
 	{
 		const bool ok = j + lane < n;
