@@ -204,3 +204,30 @@ def test_dd_psf_histogram_quads_equal_scalar(dims, lengths, mrd):
     # The weights differ by the rounding of tap coordinates counted from
     # another voxel (2 ulp of up to 18 taps, 0.25 of a tap's weight each).
     assert float((quads - scalar).norm() / scalar.norm()) < 3e-6
+
+
+# An EM ratio that overflows reaches the voxels its line crosses, as in the
+# scalar form, not the rest of their float4 groups.
+@pytest.mark.parametrize("ratio", [np.inf, np.nan])
+def test_dd_psf_histogram_quads_keep_infinite_ratios_on_their_lines(ratio):
+    sc = yrt.Scanner("t", 40, 4, 4, 10, 100, 48, 6, 1, 4, 3, 1)
+    ip = yrt.ImageParams(40, 36, 12, 160.0, 150.0, 40.0)
+    pp = yrt.ProjectorParams(sc)
+    pp.setProjector("DD")
+    pp.precision = L.YRTB_COMPENSATED
+    k = np.exp(-0.5 * ((np.arange(9) - 4) * 0.6 / 1.2) ** 2)
+    pp.setProjPsf(300.0, 0.6, (k / (k.sum() * 0.6)).astype(np.float32)[None])
+    p = yrt.DeviceProjector(sc, ip, pp)
+    h = yrt.Histogram3D(sc)
+    x = torch.full(ip.shape, 1e-30, device="cuda")
+    for b in range(7, h.histoSize, h.histoSize // 40):  # lines along both axes
+        meas = torch.zeros(h.histoSize, device="cuda")
+
+        def em(m):
+            meas[b] = m
+            return p.em_step_histo3d(x, torch.zeros(ip.shape, device="cuda"), meas, 1, 0)
+
+        on_line = em(1.0) != 0
+        # 1e38 / 1e-28 overflows.
+        bad = ~em(1e38 if np.isinf(ratio) else np.nan).isfinite()
+        assert torch.equal(bad, on_line)
