@@ -1,12 +1,16 @@
 """Image-space PSF on the device (yrtb_psf_*, OperatorPsfDevice) and OSEM
 with an image-space PSF, against the reference OperatorPsf and OSEM_CPU
 (src/operators/OperatorPsf.cpp:288-375, src/recon/OSEM_CPU.cpp:150-230)."""
+import ctypes
+import threading
+
 import numpy as np
 import pytest
 import torch
 
 import pyoracle as po
 import pyyrtpet_b200 as yrt
+from pyyrtpet_b200 import _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -369,3 +373,56 @@ def test_varpsf_tiles_vs_taps(shape, half, gaps):
     # n positive FP32 terms: at most n roundings of half an ulp of the sum.
     n = int(np.prod([2 * h + 1 for h in half]))
     assert rel_l2(adj, want) < max(2, n) * 2.0 ** -24
+
+
+def _in_threads(*calls):
+    """Each call(stream) many times, in a thread and on a stream of its own, all
+    at once; library calls without Python around them, so that they overlap."""
+    bad = []
+    start = threading.Barrier(len(calls))
+
+    def work(call):
+        stream = torch.cuda.Stream()
+        start.wait()
+        for _ in range(10000):
+            if call(stream.cuda_stream):
+                bad.append(call)
+
+    threads = [threading.Thread(target=work, args=(c,)) for c in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not bad, f"{len(bad)} failed launches"
+
+
+# The kernels' shared memory differs from call to call; their limit is set for
+# the process.
+def test_varpsf_from_two_threads():
+    def apply(half):
+        ip = yrt.ImageParams(32, 32, 8, 64.0, 64.0, 16.0)
+        op = yrt.OperatorVarPsfDevice(ip)
+        op.setKernelCollection([np.ones([2 * half + 1] * 3, np.float32)])
+        op.setRangeAndGap(32.0, 64.0, 32.0, 64.0, 8.0, 16.0)
+        x = torch.rand(ip.shape, device="cuda")
+        out = torch.empty_like(x)
+        op.applyA(x, out, ip)
+        torch.cuda.synchronize()
+        f, c = L.lib().yrtb_varpsf_apply, ip._c()
+        args = (op.handle, x.data_ptr(), out.data_ptr(), ctypes.byref(c), 0)
+        return lambda stream, keep=(op, x, out, c): f(*args, stream)
+
+    _in_threads(apply(1), apply(3), apply(1), apply(3))
+
+
+def test_low_rank_contraction_from_two_threads():
+    def contract(R, T):
+        W, E = (torch.rand(n, 256, device="cuda") for n in (R, T))
+        out = torch.empty(R, T, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        f = L.lib().yrtb_lr_contract_h
+        args = (W.data_ptr(), E.data_ptr(), R, T, 256, out.data_ptr())
+        return lambda stream, keep=(W, E, out): f(*args, stream)
+
+    _in_threads(contract(4, 120), contract(4, 400))

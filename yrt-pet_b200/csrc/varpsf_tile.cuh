@@ -59,6 +59,7 @@ constexpr int kVarMaxSeg = 48;   // segments of the x axis in the launch paramet
 constexpr int kVarMaxHx = 8;     // largest half size along x of the register window
 constexpr int kVarOut = 8;       // outputs per thread
 constexpr int kVarTileX = 32, kVarTileY = 32, kVarThreads = 256;
+constexpr size_t kVarMaxShared = 113 * 1024;  // two blocks per SM
 
 // Segments of constant LUT coordinate along one axis, of the circular axis
 // unrolled to [-H, n + H): segment s covers [start[s], start[s + 1]) and holds

@@ -5368,15 +5368,18 @@ yrtb_status yrtb_lr_contract_h(const float* d_W, const float* d_E, int R, int T,
 	// The voxel tile, or the threads' four FP64 sums if those are larger.
 	const size_t smem = std::max(static_cast<size_t>(R + T) * (kLrTile + 1) * sizeof(float),
 	                             static_cast<size_t>(kLrBlock) * 4 * sizeof(double));
-	if (P > kLrPairs * kLrBlock || smem > 227 * 1024)
+	constexpr size_t kMaxShared = 227 * 1024;
+	if (P > kLrPairs * kLrBlock || smem > kMaxShared)
 		return fail(YRTB_ERR_ARGUMENT,
 		            "low-rank basis too large for the H contraction "
 		            "(rank x frames <= 2048, rank + frames <= 440)");
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+	// The limit belongs to the kernel, not to this call: always the largest, so
+	// that calls of other threads never lower it before a launch.
 	if (smem > 48 * 1024)
 		YRTB_CUDA(cudaFuncSetAttribute(k_lr_contract_h,
 		                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                               static_cast<int>(smem)));
+		                               static_cast<int>(kMaxShared)));
 	const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>(
 	    (J + kLrTile - 1) / kLrTile, static_cast<uint64_t>(gridFor(1 << 30, kLrBlocksPerSM))));
 	double* partial = nullptr;
@@ -5608,12 +5611,11 @@ static bool varTileFits(const yrtb_varpsf* p, const VarPsfDev& P, const int* dim
 	// leaves SMs without a block, at least 2 (8 warps, 4 chunks per plane).
 	const int64_t cols = static_cast<int64_t>((T.chunks + 3) / 4) *
 	                     ((dims[1] + kVarTileY - 1) / kVarTileY);
-	constexpr size_t kTwoPerSM = 113 * 1024;
 	for (T.zt = 8;; T.zt /= 2)
 	{
 		T.zTiles = (dims[2] + T.zt - 1) / T.zt;
 		const int64_t blocks = cols * T.zTiles * nt;
-		if (varShared(T) <= kTwoPerSM &&
+		if (varShared(T) <= kVarMaxShared &&
 		    (T.zt == 2 || blocks >= 4 * static_cast<int64_t>(gridFor(1u << 30, 1))))
 			return T.zTiles * nt <= 65535;
 		if (T.zt == 2)
@@ -5674,8 +5676,9 @@ yrtb_status yrtb_varpsf_apply(const yrtb_varpsf* p, const float* d_in, float* d_
 		                 static_cast<unsigned>(T.zTiles * ip->nt));
 		auto go = [&](auto kernel) -> yrtb_status
 		{
+			// The kernel's limit, not this call's size: see yrtb_lr_contract_h.
 			YRTB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                               static_cast<int>(shared)));
+			                               static_cast<int>(kVarMaxShared)));
 			kernel<<<tiles, kVarThreads, shared, st>>>(d_in, d_out, dims[0], dims[1], dims[2], T);
 			YRTB_LAUNCHED();
 			return YRTB_OK;
