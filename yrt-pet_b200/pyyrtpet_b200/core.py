@@ -934,9 +934,20 @@ class DeviceProjector:
             _ptr(mu), mp, int(num_subsets), int(subset), _stream()))
         return sens_img
 
+    def _check_bins(self, values: torch.Tensor, img: torch.Tensor):
+        """values: one float32 per bin of the projector's histogram, beside img."""
+        if not (values.is_cuda and values.dtype == torch.float32 and values.is_contiguous()):
+            raise RuntimeError("bin values must be a contiguous float32 CUDA tensor")
+        if values.device != img.device:
+            raise RuntimeError(f"bin values on {values.device}, image on {img.device}")
+        want = Histogram3D(self.scanner).histoSize
+        if values.numel() != want:
+            raise RuntimeError(f"{values.numel()} bin values, expected {want}")
+
     def forward_histo3d(self, img, values, num_subsets=1, subset=0):
         """values[bin] = A img over one subset of the histogram's bins."""
         self._check_image(img)
+        self._check_bins(values, img)
         L.check(L.lib().yrtb_forward_histo3d(self.h, img.data_ptr(), int(num_subsets),
                                              int(subset), values.data_ptr(), _stream()))
         return values
@@ -944,6 +955,7 @@ class DeviceProjector:
     def backward_histo3d(self, values, img, num_subsets=1, subset=0):
         """img += A^T values over one subset of the histogram's bins."""
         self._check_image(img)
+        self._check_bins(values, img)
         L.check(L.lib().yrtb_backward_histo3d(self.h, values.data_ptr(), int(num_subsets),
                                               int(subset), img.data_ptr(), _stream()))
         return img
@@ -1137,17 +1149,18 @@ class OperatorProjectorDevice:
         raise RuntimeError("The Projection Data provided is not a "
                            "ProjectionList, ListModeLUT nor Histogram3D")
 
-    def _whole_histogram(self, projData, vals, p: DeviceProjector) -> bool:
+    def _whole_histogram(self, projData, vals, img, p: DeviceProjector) -> bool:
         """Whether the bins of the iterator can be projected from their index
         (forward_histo3d): a subset of the projector's own histogram and one
-        float32 value per bin.  Other iterators, scanners and value arrays go
+        float32 value per bin on the image's device.  Other iterators, scanners and value arrays go
         through lists of bins and crystal pairs."""
         it, h = self.bin_iter, projData
         return (isinstance(h, Histogram3D) and type(it) is BinIteratorRangeHistogram3D
                 and h.scanner is p.scanner
                 and (it.numZBin, it.numPhi, it.numR) == (h.numZBin, h.numPhi, h.numR)
                 and 0 <= it.idxSubset < it.numSubsets
-                and vals.is_cuda and vals.dtype == torch.float32 and vals.is_contiguous()
+                and vals.is_cuda and vals.device == img.device
+                and vals.dtype == torch.float32 and vals.is_contiguous()
                 and vals.dim() == 1 and vals.numel() == h.histoSize
                 and not vals.requires_grad
                 and p.get_image_layout() == L.YRTB_LAYOUT_ROW_MAJOR)
@@ -1167,7 +1180,7 @@ class OperatorProjectorDevice:
         p = self._projector()
         self._check_image(img, p)
         vals = proj._require()
-        if self._whole_histogram(proj.reference, vals, p):
+        if self._whole_histogram(proj.reference, vals, img, p):
             p.forward_histo3d(img.contiguous(), vals, self.bin_iter.numSubsets,
                               self.bin_iter.idxSubset)
             return proj
@@ -1187,7 +1200,7 @@ class OperatorProjectorDevice:
         p = self._projector()
         self._check_image(img, p)
         vals = proj._require()
-        if self._whole_histogram(proj.reference, vals, p):
+        if self._whole_histogram(proj.reference, vals, img, p):
             return p.backward_histo3d(vals, img, self.bin_iter.numSubsets,
                                       self.bin_iter.idxSubset)
         ev, rng = self._events(proj)
