@@ -320,3 +320,80 @@ def test_small_launches_equal_the_set_shape(precision, tof, n):
     assert a[4] == b[4]
     for i in (2, 3):  # the same terms, added in another order
         assert rel_l2(a[i].cpu().numpy(), b[i].cpu().numpy()) < 2 * n ** 0.5 * 2.0 ** -24
+
+
+def launched_blocks(call):
+    """Threads per block of the kernels that call launches (captured, not run)."""
+    from cuda.bindings import driver as cu
+
+    def ok(r):
+        assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+        return r[1:]
+
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        ok(cu.cuStreamBeginCapture(stream.cuda_stream,
+                                   cu.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_RELAXED))
+        try:
+            call()
+        finally:
+            r = cu.cuStreamEndCapture(stream.cuda_stream)
+    graph = ok(r)[0]
+    count = ok(cu.cuGraphGetNodes(graph))[1]
+    out = []
+    for node in ok(cu.cuGraphGetNodes(graph, count))[0]:
+        if ok(cu.cuGraphNodeGetType(node))[0] == cu.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            out.append(int(ok(cu.cuGraphKernelNodeGetParams(node))[0].blockDimX))
+    ok(cu.cuGraphDestroy(graph))
+    return out
+
+
+# One-warp blocks for small launches and forward projections, as long as no shape
+# was set; a shape that was set is the one that runs.
+@pytest.mark.parametrize("precision", [L.YRTB_MIRROR, L.YRTB_COMPENSATED])
+@pytest.mark.parametrize("tof", [None, (214.0, 5)])
+def test_a_set_shape_is_launched(precision, tof):
+    sc, ip, p = make(tof, precision)
+    d1, d2 = random_events(5000, 63)
+    tv = np.zeros(len(d1), np.float32) if tof else None
+    ev = yrt.DeviceEvents.from_arrays(d1, d2, tof=tv)
+    x = torch.ones(ip.shape, device="cuda")
+    y, img = torch.ones(len(d1), device="cuda"), torch.zeros_like(x)
+    calls = [lambda: p.forward(x, ev, out=y), lambda: p.backward(y, ev, img=img),
+             lambda: p.em_step(x, img, ev)]
+    assert [launched_blocks(c) for c in calls] == [[32]] * 3
+    for block in (128, 256):
+        for groups in (0, 2, 8):
+            p.set_launch(block, 1, 3, vector_groups=groups)
+            assert [launched_blocks(c) for c in calls] == [[block]] * 3
+    default = yrt.DeviceProjector(sc, ip, p.proj_params).get_launch()
+    p.set_launch(**default)
+    assert [launched_blocks(c) for c in calls] == [[default["block"]]] * 3
+
+
+def test_autotune_that_fails_leaves_the_launch_shape_unset():
+    sc, ip, p = make((214.0, 5))
+    d1, d2 = random_events(5000, 64)
+    ev = yrt.DeviceEvents.from_arrays(d1, d2, tof=np.zeros(len(d1), np.float32))
+    x, y = torch.ones(ip.shape, device="cuda"), torch.ones(len(d1), device="cuda")
+    img = torch.zeros_like(x)
+    before = p.get_launch()
+
+    def tune():
+        # A captured event has no time: the first measurement fails.
+        with pytest.raises(yrt.YrtbError):
+            p.autotune(x, ev)
+
+    try:
+        launched_blocks(tune)
+    except AssertionError:
+        pass  # the capture may be lost with it
+    try:
+        p.backward(y, ev, img=img)
+    except yrt.YrtbError:
+        pass  # what the lost capture left for the next launch's check
+    assert p.get_launch() == before
+    assert launched_blocks(lambda: p.backward(y, ev, img=img)) == [32]
+    p.autotune(x, ev)
+    assert launched_blocks(lambda: p.backward(y, ev, img=img)) == [p.get_launch()["block"]]

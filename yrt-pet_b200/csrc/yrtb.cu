@@ -3140,7 +3140,7 @@ struct yrtb_projector
 	uint64_t mrCapacity = 0;
 	// Launch configuration of the single-ray Siddon event kernels.
 	yrtb_launch_config launch{256, 1, 3, YRTB_ORDER_LOR, 1, 2};
-	// Set by the caller (yrtb_projector_set_launch) or the autotuner.
+	// Set by the caller (yrtb_projector_set_launch) or chosen by the autotuner.
 	bool launchSet = false;
 	// Layout of the images of the list-mode projections (YRTB_LAYOUT_*).
 	int layout = YRTB_LAYOUT_ROW_MAJOR;
@@ -3532,9 +3532,7 @@ yrtb_status dispatchEvents(yrtb_projector* h, const yrtb_events* ev,
 			{
 				// The small form replaces the default launch shape only: one
 				// that was set is kept.
-				if (!tiled && R.count <= smallEvents<OP, T, C>() &&
-				    h->launch.threads_per_lor == 1 &&
-				    (OP == OP_FWD ? !(h->launch.vector_groups & 1) : !h->launchSet))
+				if (!tiled && R.count <= smallEvents<OP, T, C>() && !h->launchSet)
 				{
 					k_events_batch<OP, T, C>
 					    <<<static_cast<unsigned>((R.count + kSmallBlock - 1) / kSmallBlock),
@@ -5953,6 +5951,7 @@ yrtb_status yrtb_autotune(yrtb_projector* h, const float* d_image,
 	cudaMemsetAsync(em, 0, J * 4, st);
 
 	const yrtb_launch_config saved = h->launch;
+	const bool savedSet = h->launchSet;
 	h->launchSet = true;  // the configurations are timed as they are
 	cudaEvent_t e0 = nullptr, e1 = nullptr;
 	cudaEventCreate(&e0);
@@ -6053,6 +6052,7 @@ yrtb_status yrtb_autotune(yrtb_projector* h, const float* d_image,
 	cudaEventDestroy(e1);
 	release();
 	h->launch = bestIdx >= 0 ? report->tried[bestIdx] : saved;
+	h->launchSet = savedSet || bestIdx >= 0;
 	report->best = h->launch;
 	report->sample_events = n;
 	if (s != YRTB_OK)
