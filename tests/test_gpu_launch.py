@@ -397,3 +397,64 @@ def test_autotune_that_fails_leaves_the_launch_shape_unset():
     assert launched_blocks(lambda: p.backward(y, ev, img=img)) == [32]
     p.autotune(x, ev)
     assert launched_blocks(lambda: p.backward(y, ev, img=img)) == [p.get_launch()["block"]]
+
+
+def kept_after(use):
+    """Bytes of device memory that use() still holds once all it made is gone."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    yrt.release_cached_memory()
+    before = torch.cuda.mem_get_info()[0]
+    use()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return before - torch.cuda.mem_get_info()[0]
+
+
+# The library's pool keeps at most small tables of a projector that is gone.
+def test_large_tables_go_with_the_projector():
+    sc, ip, _ = make()
+    pp = yrt.ProjectorParams(sc)
+    pp.numRays = 3
+
+    def table():
+        p = yrt.DeviceProjector(sc, ip, pp)
+        p.multiray_table(1 << 20)    # 32 MB: pool
+        p.multiray_table(1 << 23)    # 256 MB
+        p.multiray_table(1 << 23)    # large enough already
+        assert torch.equal(p.multiray_offsets(5), yrt.DeviceProjector(sc, ip, pp).multiray_offsets(5))
+
+    assert kept_after(table) <= 64 << 20
+
+
+def test_stored_sensitivity_values_go_with_the_projector():
+    # 33M bins: 132 MB of values between the two passes.
+    sc = yrt.Scanner("t", 100, 4, 3, 10, 250, 400, 20, 1, 19, 1, 1)
+    ip = yrt.ImageParams(24, 24, 12, 240.0, 240.0, 90.0)
+    assert yrt.Histogram3D(sc).histoSize * 4 > 64 << 20
+    pp = yrt.ProjectorParams(sc)
+    pp.deterministic = True
+    mu = torch.rand(ip.shape, device="cuda") * 0.01
+    out = {}
+
+    def image(name, captured):
+        p = yrt.DeviceProjector(sc, ip, pp)
+        img = torch.zeros(ip.shape, device="cuda")
+        torch.cuda.synchronize()
+        call = lambda: p.sensitivity_histo3d(img, mu=mu, mu_params=ip)
+        if captured:
+            # A captured call holds no such buffer: both passes walk.
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                call()
+            g.replay()
+        else:
+            call()
+            img.zero_()
+            call()
+        torch.cuda.synchronize()
+        out[name] = img.cpu()
+
+    assert kept_after(lambda: image("stored", False)) <= 64 << 20
+    image("walked", True)
+    assert float(out["stored"].norm()) > 0 and torch.equal(out["stored"], out["walked"])

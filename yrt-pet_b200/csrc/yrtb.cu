@@ -3151,20 +3151,44 @@ struct yrtb_projector
 	int device = 0;
 
 	// Tables of at most kPooledBytes come from the library's pool (no driver
-	// allocation per projector), larger ones from cudaMalloc.
+	// allocation per projector), larger ones from cudaMalloc, so that what the
+	// pool keeps after the projector is bounded.
 	static constexpr size_t kPooledBytes = size_t(64) << 20;
 	std::vector<void*> pooled, owned;
+	// Bin values kept between the passes of a deterministic sensitivity image,
+	// where they are too many for the pool (used like d_fix by one call at a
+	// time).
+	float* d_stored = nullptr;
+	uint64_t storedCapacity = 0;
 
+	// st: the stream of the table's first use.
 	template <typename T>
-	cudaError_t make(T** p, size_t count)
+	cudaError_t make(T** p, size_t count, cudaStream_t st = nullptr)
 	{
 		const size_t bytes = std::max<size_t>(1, count * sizeof(T));
 		const bool pool = bytes <= kPooledBytes;
-		const cudaError_t e = pool ? poolAlloc(p, bytes, nullptr)
+		const cudaError_t e = pool ? poolAlloc(p, bytes, st)
 		                           : cudaMalloc(reinterpret_cast<void**>(p), bytes);
 		if (e == cudaSuccess)
 			(pool ? pooled : owned).push_back(*p);
 		return e;
+	}
+
+	// Gives a table of make back; no launch may use it any more.
+	template <typename T>
+	cudaError_t drop(T** p, cudaStream_t st)
+	{
+		void* old = *p;
+		*p = nullptr;
+		for (auto* list : {&pooled, &owned})
+		{
+			const auto at = std::find(list->begin(), list->end(), old);
+			if (at == list->end())
+				continue;
+			list->erase(at);
+			return list == &pooled ? cudaFreeAsync(old, st) : cudaFree(old);
+		}
+		return cudaSuccess;
 	}
 
 	~yrtb_projector()
@@ -3180,8 +3204,6 @@ struct yrtb_projector
 		{
 			for (void* p : pooled)
 				cudaFreeAsync(p, nullptr);
-			if (d_mrTable)
-				cudaFreeAsync(d_mrTable, nullptr);
 		}
 		for (void* p : owned)
 			cudaFree(p);
@@ -3608,6 +3630,46 @@ struct NonzeroBin
 // sensitivity image; larger subsets walk the attenuation image in both.
 constexpr uint64_t kStoredBytes = uint64_t(512) << 20;
 
+// Room for count bin values: from the pool for this call, or the projector's
+// own buffer above kPooledBytes.  Null if there is none, or while the stream is
+// captured: a graph would hold the allocation, or a pointer that a later call
+// gives back.
+float* storedValues(yrtb_projector* h, uint64_t count, cudaStream_t st)
+{
+	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+	if (count * sizeof(float) > kStoredBytes ||
+	    cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
+	    capture != cudaStreamCaptureStatusNone)
+	{
+		(void)cudaGetLastError();
+		return nullptr;
+	}
+	float* p = nullptr;
+	cudaError_t e = cudaSuccess;
+	if (count * sizeof(float) <= yrtb_projector::kPooledBytes)
+	{
+		e = poolAlloc(&p, count * sizeof(float), st);
+	}
+	else
+	{
+		if (count > h->storedCapacity)
+		{
+			h->storedCapacity = 0;
+			// (cudaFree waits for the launches that use it.)
+			e = h->drop(&h->d_stored, st);
+			if (e == cudaSuccess)
+				e = h->make(&h->d_stored, count);
+			if (e == cudaSuccess)
+				h->storedCapacity = count;
+		}
+		p = h->d_stored;
+	}
+	if (e == cudaSuccess)
+		return p;
+	(void)cudaGetLastError();
+	return nullptr;
+}
+
 // Runs one histogram operation over a subset's bins, or the listed ones.  A
 // holds the operation's buffers; the subset and the two-pass fields are set
 // here.
@@ -3649,12 +3711,8 @@ yrtb_status dispatchHisto(yrtb_projector* h, int numSubsets, int subset, HistoAr
 			return s;
 		// Pass 1 keeps the values whose attenuation it walked for pass 2; with
 		// no room for them, pass 2 walks again.
-		if (HOP == HOP_SENS && A.muImg && !A.acfH && A.count * sizeof(float) <= kStoredBytes &&
-		    poolAlloc(&A.stored, A.count * sizeof(float), st) != cudaSuccess)
-		{
-			A.stored = nullptr;
-			(void)cudaGetLastError();
-		}
+		if (HOP == HOP_SENS && A.muImg && !A.acfH)
+			A.stored = storedValues(h, A.count, st);
 	}
 	auto launch = [&](auto kind, auto comp)
 	{
@@ -3738,7 +3796,7 @@ yrtb_status dispatchHisto(yrtb_projector* h, int numSubsets, int subset, HistoAr
 	}
 	if (det)
 	{
-		if (A.stored)
+		if (A.stored && A.stored != h->d_stored)
 			cudaFreeAsync(A.stored, st);
 		fixedEnd(h, A.F, A.out, st);
 	}
@@ -4398,12 +4456,10 @@ yrtb_status yrtb_multiray_table(yrtb_projector* h, uint64_t count,
 		h->P.mrTable = nullptr;
 		h->P.mrCount = 0;
 		h->mrCapacity = 0;
-		float* old = h->d_mrTable;
-		h->d_mrTable = nullptr;
-		YRTB_CUDA(cudaFreeAsync(old, st));
+		YRTB_CUDA(h->drop(&h->d_mrTable, st));
 	}
 	const uint64_t per = 4 * static_cast<uint64_t>(h->P.numRays - 1);
-	YRTB_CUDA(poolAlloc(&h->d_mrTable, count * per * sizeof(float), st));
+	YRTB_CUDA(h->make(&h->d_mrTable, count * per, st));
 	k_multiray_offsets<<<gridAll((count + kMrItems - 1) / kMrItems), kBlock, 0, st>>>(
 	    count, h->P.numRays, h->d_mrTable);
 	YRTB_LAUNCHED();
