@@ -458,3 +458,24 @@ def test_stored_sensitivity_values_go_with_the_projector():
     assert kept_after(lambda: image("stored", False)) <= 64 << 20
     image("walked", True)
     assert float(out["stored"].norm()) > 0 and torch.equal(out["stored"], out["walked"])
+
+
+def test_multi_ray_table_is_not_made_under_capture():
+    sc, ip, _ = make()
+    pp = yrt.ProjectorParams(sc)
+    pp.numRays = 3
+    p = yrt.DeviceProjector(sc, ip, pp)
+
+    def make_table(count):
+        with pytest.raises(yrt.YrtbError, match="captured"):
+            p.multiray_table(count)
+
+    assert launched_blocks(lambda: make_table(100)) == []
+    p.multiray_table(100)
+    assert launched_blocks(lambda: p.multiray_table(50)) == []  # large enough already
+    assert launched_blocks(lambda: make_table(200)) == []
+    d1, d2 = random_events(200, 65)
+    ev = yrt.DeviceEvents.from_arrays(d1, d2)
+    x = torch.rand(ip.shape, device="cuda")
+    # The first table still serves; item 100 on derive their offsets.
+    assert torch.equal(p.forward(x, ev), yrt.DeviceProjector(sc, ip, pp).forward(x, ev))

@@ -3626,6 +3626,16 @@ struct NonzeroBin
 	}
 };
 
+// Whether st is being captured (or cannot say).
+bool capturing(cudaStream_t st)
+{
+	cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(st, &s) == cudaSuccess)
+		return s != cudaStreamCaptureStatusNone;
+	(void)cudaGetLastError();
+	return true;
+}
+
 // Largest array of bin values kept between the two passes of a deterministic
 // sensitivity image; larger subsets walk the attenuation image in both.
 constexpr uint64_t kStoredBytes = uint64_t(512) << 20;
@@ -3636,14 +3646,8 @@ constexpr uint64_t kStoredBytes = uint64_t(512) << 20;
 // gives back.
 float* storedValues(yrtb_projector* h, uint64_t count, cudaStream_t st)
 {
-	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-	if (count * sizeof(float) > kStoredBytes ||
-	    cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
-	    capture != cudaStreamCaptureStatusNone)
-	{
-		(void)cudaGetLastError();
+	if (count * sizeof(float) > kStoredBytes || capturing(st))
 		return nullptr;
-	}
 	float* p = nullptr;
 	cudaError_t e = cudaSuccess;
 	if (count * sizeof(float) <= yrtb_projector::kPooledBytes)
@@ -4449,6 +4453,10 @@ yrtb_status yrtb_multiray_table(yrtb_projector* h, uint64_t count,
 		return YRTB_OK;
 	YRTB_CUDA(cudaSetDevice(h->device));
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+	// Captured, the table would be the graph's: without memory until the graph
+	// runs, and the projector would read it in any later call.
+	if (capturing(st))
+		return fail(YRTB_ERR_CUDA, "the multi-ray table cannot be made while a stream is captured");
 	if (h->d_mrTable)
 	{
 		// Launches already queued may still read the old table.
