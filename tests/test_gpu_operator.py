@@ -219,15 +219,62 @@ def test_dd_psf_histogram_quads_keep_infinite_ratios_on_their_lines(ratio):
     pp.setProjPsf(300.0, 0.6, (k / (k.sum() * 0.6)).astype(np.float32)[None])
     p = yrt.DeviceProjector(sc, ip, pp)
     h = yrt.Histogram3D(sc)
-    x = torch.full(ip.shape, 1e-30, device="cuda")
+    n = ip.numVoxels
+    x = torch.full((n + 1,), 1e-30, device="cuda")
     for b in range(7, h.histoSize, h.histoSize // 40):  # lines along both axes
         meas = torch.zeros(h.histoSize, device="cuda")
 
-        def em(m):
+        def em(m, first):  # first = 1: the scalar form
             meas[b] = m
-            return p.em_step_histo3d(x, torch.zeros(ip.shape, device="cuda"), meas, 1, 0)
+            buf = torch.zeros(n + 1, device="cuda")
+            p.em_step_histo3d(x[first:first + n], buf[first:first + n], meas, 1, 0)
+            return buf[first:first + n]
 
-        on_line = em(1.0) != 0
         # 1e38 / 1e-28 overflows.
-        bad = ~em(1e38 if np.isinf(ratio) else np.nan).isfinite()
-        assert torch.equal(bad, on_line)
+        m = 1e38 if np.isinf(ratio) else np.nan
+        bad = ~em(m, 0).isfinite()
+        assert torch.equal(bad, ~em(m, 1).isfinite())
+        # The whole line (and voxels that its rows end in with weight 0).
+        assert bool(bad[em(1.0, 1) != 0].all()) and not bad.all()
+
+
+def test_dd_psf_weights_are_as_exact_as_their_arithmetic():
+    # Lines along x, so that a footprint's edges are FP32 numbers known here, on
+    # voxels whose edges are whole: what rounds is the integral of the kernel
+    # (4 mm FWHM, taps of 0.5 mm) over each voxel.
+    sc = yrt.Scanner("t", 8, 2, 1, 10, 200, 16, 1, 1, 0, 1, 1)
+    ip = yrt.ImageParams(4, 48, 1, 4.0, 48.0, 8.0)
+    pp = yrt.ProjectorParams(sc)
+    pp.setProjector("DD")
+    pp.precision = L.YRTB_COMPENSATED
+    half, step = 11, 0.5
+    g = np.exp(-0.5 * (np.arange(-half, half + 1) * step * 2.3548 / 4.0) ** 2)
+    taps = (g / (g.sum() * step)).astype(np.float32)
+    pp.setProjPsf(1e9, step, taps[None])
+    p = yrt.DeviceProjector(sc, ip, pp)
+    n = 4000
+    y = np.random.default_rng(71).uniform(-20, 20, n).astype(np.float32)
+    lor, orient = np.zeros((n, 6), np.float32), np.zeros((n, 6), np.float32)
+    lor[:, 0], lor[:, 3], lor[:, 1], lor[:, 4] = 200, -200, y, y
+    orient[:, 0], orient[:, 3] = 1, -1
+    ev = yrt.DeviceEvents.from_arrays(lor=lor, orient=orient)
+    offs, wts, cnt = (t.cpu().numpy() for t in p.trace_walks(ev, cap=256))
+    near, far = (y - np.float32(0.5)).astype(np.float64), (y + np.float32(0.5)).astype(np.float64)
+
+    def integral(x):  # of the taps' polygon from far left to x mm from the centre
+        v = np.concatenate([[0, 0], taps.astype(np.float64), [0]])
+        whole = np.concatenate([[0, 0], np.cumsum((v[2:] + v[1:-1]) * step / 2)])
+        u = np.clip(x / step, -half - 1, half + 1)
+        i = np.minimum(np.floor(u).astype(int), half) + half + 2
+        t = u - (i - half - 2)
+        return whole[i] + step * (v[i] * t + (v[np.minimum(i + 1, len(v) - 1)] - v[i]) * t * t / 2)
+
+    on = np.arange(offs.shape[1])[None] < cnt[:, None]
+    assert on.sum(1).min() > 40
+    edge = (offs // 4 - 24).astype(np.float64)
+    want = (integral(edge + 1 - near[:, None]) - integral(edge - far[:, None]))[on]
+    got = (wts.astype(np.float64) * (far - near)[:, None])[on]  # rows 1 mm long, one plane
+    assert want.max() > 0.2
+    # About four roundings of a weight (its parts, their sum, the row's factor):
+    # half an ulp at random, 2^-25 to 2^-24 of it.
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < 2 * 2.0 ** -24.5 / 3 ** 0.5

@@ -49,8 +49,8 @@ struct Psf
 	const float* flipped;  // adjoint taps
 	int num_s, size;
 	float sStep, kSpacing;
-	// Integral of each kernel row as a piecewise parabola (num_s * (size + 2)
-	// pieces, see psfCdf), of the taps and of the flipped taps.
+	// Integral of each kernel row as a piecewise parabola (size + 2 pieces and
+	// the whole, see psfCdf), of the taps and of the flipped taps.
 	const float4* cdf;
 	const float4* cdfFlipped;
 };
@@ -973,25 +973,34 @@ __device__ __forceinline__ float psfIntegral(const float* kernel,
 
 // The integral of the same kernel as a table: the kernel is linear between its
 // taps, so its integral is a parabola on each of the size + 1 pieces between
-// them (u = 0 .. size + 1, in steps from one step before the first tap; smaller
-// and larger u are clamped), q = {value at the piece's start, first and second
-// coefficient}.  Pieces before the centre tap hold the integral from the left
+// them, q = {value at the piece's start, first and second coefficient, rest of
+// the value}.  Pieces before the centre tap hold the integral from the left
 // end, pieces from it on minus the integral to the right end, so that both
 // tails keep their relative precision: the integral from a to b is cdf(b) -
-// cdf(a), plus the whole (first entry's w) if the centre lies between them.
-// (Measured from the left end throughout, the weights in the right tail lost
-// five digits, and an image whose lines see only tails was 1.2e-5 from 64 bits
-// instead of 1.7e-6.)  One 16-byte read and two fused multiply-adds, where
-// the bins' form takes about 60 instructions.  A NaN u counts as 0.
-__device__ __forceinline__ float psfCdf(const float4* __restrict__ cdf, float top, float u)
+// cdf(a), plus the whole (one entry past the pieces, in the same two parts) if
+// the centre lies between them.  (Measured from the left end throughout, the
+// weights in the right tail lost five digits, and an image whose lines see
+// only tails was 1.2e-5 from 64 bits instead of 1.7e-6.)  The values' first
+// parts are multiples of 2^-22 of the largest, so that they subtract and add
+// without rounding, and what rounds is of the size of a piece.  Voxels and
+// crystals of 1 mm, a kernel of 4 mm in taps of 0.5 mm: integrals 2.5e-8 from 64
+// bits, 8.9e-8 with single values and taps counted from the left end, 8.7e-8
+// summed by bins.
+//
+// u: taps from the centre, clamped to [lo, hi], one step beyond the first and
+// the last tap.  biased: address of the centre tap's piece less kCdfBias
+// pieces.  One 16-byte read and two fused multiply-adds, where the bins' form
+// takes about 60 instructions.  A NaN u counts as lo.
+constexpr int kCdfBias = 0x4b400000;  // bits of 1.5 * 2^23
+__device__ __forceinline__ float2 psfCdf(uint64_t biased, float lo, float hi, float u)
 {
-	u = fminf(fmaxf(u, 0.f), top);
+	u = fminf(fmaxf(u, lo), hi);
 	// Integer part by an addition that rounds down into the low mantissa bits.
-	const float f = __fadd_rd(u, 8388608.f);
-	const int i = __float_as_int(f) & 0x7fffff;
-	const float t = u - (f - 8388608.f);
-	const float4 q = __ldg(cdf + i);
-	return __fmaf_rn(t, __fmaf_rn(t, q.z, q.y), q.x);
+	const float f = __fadd_rd(u, __int_as_float(kCdfBias));
+	const float t = u - (f - __int_as_float(kCdfBias));
+	const float4 q = __ldg(reinterpret_cast<const float4*>(
+	    biased + sizeof(float4) * static_cast<uint64_t>(__float_as_uint(f))));
+	return make_float2(q.x, __fmaf_rn(t, __fmaf_rn(t, q.z, q.y), q.w));
 }
 
 // Distance-driven footprint of one LOR.  d1, d2: crystal centres relative to
@@ -1299,7 +1308,7 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 			s_idx = (si >= static_cast<float>(psf.num_s - 1)) ? psf.num_s - 1 :
 			                                                    static_cast<int>(si);
 		}
-		cdf = (forward ? psf.cdf : psf.cdfFlipped) + s_idx * (psf.size + 2);
+		cdf = (forward ? psf.cdf : psf.cdfFlipped) + s_idx * (psf.size + 3);
 		ext = static_cast<float>((psf.size + 1) / 2) * psf.kSpacing;
 	}
 	const float dx = g.vx, dy = g.vy, dz = g.vz;
@@ -1399,10 +1408,14 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 	const float r_z_hi = 1.0f / (d2_z_hi_i - d1_z_hi_i);
 	const float r_i = TOF ? 1.0f / (d2_i - d1_i) : 0.f;
 	const float r_step = 1.0f / psf.kSpacing;
-	const float top = static_cast<float>(psf.size + 1);
-	const float mid = static_cast<float>((psf.size + 1) / 2);
+	const int mid = (psf.size + 1) / 2;
+	const float lo = -static_cast<float>(mid), hi = static_cast<float>(psf.size + 1 - mid);
 	const float du = dyx * r_step;  // taps per voxel
-	const float whole = __ldg(cdf).w;
+	const float4 whole = __ldg(cdf + psf.size + 2);
+	const uint64_t biased = reinterpret_cast<uint64_t>(cdf + mid) -
+	                        sizeof(float4) * static_cast<uint64_t>(kCdfBias);
+	// Voxels from a footprint's first one to about its centre.
+	const float half = rintf(ext * inv_dyx);
 	const float y0 = -0.5f * lyx, z0 = -0.5f * g.lz;
 	// Footprint of row xyi: transverse and axial edges, and the voxels they span
 	// (false if none).
@@ -1444,11 +1457,18 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 	};
 	// Integral of the kernel over a voxel, from the tap coordinates of its
 	// near edge from the footprint's far end (ua) and of its far edge from the
-	// near end (ub); 0 outside the support.
+	// near end (ub); 0 outside the support.  Both advance by du per voxel from
+	// a voxel near the footprint's centre, where they are small.
 	auto integral = [&](float ua, float ub) -> float
 	{
-		const float w = psfCdf(cdf, top, ub) - psfCdf(cdf, top, ua);
-		return (ua < mid && ub >= mid) ? w + whole : w;
+		const float2 a = psfCdf(biased, lo, hi, ua), b = psfCdf(biased, lo, hi, ub);
+		float w = b.x - a.x, rest = b.y - a.y;
+		if (ua < 0.f && ub >= 0.f)
+		{
+			w += whole.x;
+			rest += whole.w;
+		}
+		return w + rest;
 	};
 	// Overlap of plane z0 + (zf + j) dz .. with an axial footprint, as a
 	// fraction of its width (0 if they don't meet).
@@ -1470,9 +1490,9 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 					continue;
 				const float rowW = rowWeight(rowF, R), r_wz = rcpApprox(R.z1 - R.z0);
 				const int q0 = R.i0 & ~3;
-				const float edge = y0 + static_cast<float>(q0) * dyx;
-				const float ua0 = __fmaf_rn(edge - R.r1, r_step, mid);
-				const float ub0 = __fmaf_rn(edge + dyx - R.r0, r_step, mid);
+				const float edge = y0 + (static_cast<float>(q0) + half) * dyx;
+				const float ua0 = (edge - R.r1) * r_step;
+				const float ub0 = (edge + dyx - R.r0) * r_step;
 				for (int zi = R.zi0; zi <= R.zi1; zi += kDDZ)
 				{
 					float zq[kDDZ];
@@ -1481,7 +1501,7 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 					for (int j = 0; j < kDDZ; j++)
 						zq[j] = zi + j <= R.zi1 ? axial(zf, j, R.z0, R.z1, r_wz) : 0.f;
 					int o = zi * nxy + xyi * g.nx + q0;
-					float kf = 0.f;
+					float kf = -half;
 					for (int x = q0; x <= R.i1; x += 4, kf += 4.f, o += 4)
 					{
 						float w[4];
@@ -1533,13 +1553,13 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 						zhi = max(zhi, R.zi1);
 					}
 				}
-				const float edge = y0 + static_cast<float>(ilo) * dyx;
+				const float edge = y0 + (static_cast<float>(ilo) + half) * dyx;
 				float ua0[4], ub0[4];
 #pragma unroll
 				for (int l = 0; l < 4; l++)
 				{
-					ua0[l] = __fmaf_rn(edge - rb[l], r_step, mid);
-					ub0[l] = __fmaf_rn(edge + dyx - ra[l], r_step, mid);
+					ua0[l] = (edge - rb[l]) * r_step;
+					ub0[l] = (edge + dyx - ra[l]) * r_step;
 				}
 				for (int zi = zlo; zi <= zhi; zi += kDDZ)
 				{
@@ -1551,7 +1571,7 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 						for (int l = 0; l < 4; l++)
 							zq[l][j] = axial(zf, j, z0q[l], z1q[l], rz[l]);
 					int o = zi * nxy + ilo * g.nx + 4 * q;
-					float kf = 0.f;
+					float kf = -half;
 					for (int yxi = ilo; yxi <= ihi; yxi++, kf += 1.f, o += g.nx)
 					{
 						float w[4];
@@ -1582,9 +1602,9 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 			if (!footprint(rowF, R))
 				continue;
 			const float rowW = rowWeight(rowF, R), r_wz = rcpApprox(R.z1 - R.z0);
-			const float edge = y0 + static_cast<float>(R.i0) * dyx;
-			const float ua0 = __fmaf_rn(edge - R.r1, r_step, mid);
-			const float ub0 = __fmaf_rn(edge + dyx - R.r0, r_step, mid);
+			const float edge = y0 + (static_cast<float>(R.i0) + half) * dyx;
+			const float ua0 = (edge - R.r1) * r_step;
+			const float ub0 = (edge + dyx - R.r0) * r_step;
 			const int rowO = xyi * sxy + R.i0 * syx;
 			for (int zi = R.zi0; zi <= R.zi1; zi += kDDZ)
 			{
@@ -1600,11 +1620,11 @@ __device__ __forceinline__ void ddPsfWalk(const Geom& g, const float3 d1, const 
 						zmask |= 1u << j;
 				}
 				int o = zi * nxy + rowO;
-				float kf = 0.f;
+				float kf = -half;
 				for (int yxi = R.i0; yxi <= R.i1; yxi++, kf += 1.f, o += syx)
 				{
 					const float ua = __fmaf_rn(kf, du, ua0), ub = __fmaf_rn(kf, du, ub0);
-					if (!(ua <= top && ub > 0.f))
+					if (!(ua <= hi && ub > lo))
 						continue;
 					visit(o, nxy, integral(ua, ub) * rowW, zq, zmask);
 				}

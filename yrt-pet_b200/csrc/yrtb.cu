@@ -4238,36 +4238,44 @@ yrtb_status yrtb_projector_create(const yrtb_scanner* s, const float* lut,
 		YRTB_CUDA(h->make(&h->d_flipped, n));
 		YRTB_CUDA(cudaMemcpy(h->d_taps, pp->psf_taps, n * sizeof(float), cudaMemcpyHostToDevice));
 		YRTB_CUDA(cudaMemcpy(h->d_flipped, flipped.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-		// Pieces of the integral of each kernel row (psfCdf; FP64, stored
-		// FP32): piece i runs from tap i - 1 to tap i, taps beyond the ends
-		// are 0.
-		const int K = pp->psf_size, W = K + 2;
+		// Pieces of the integral of each kernel row and the whole (psfCdf): piece
+		// i runs from tap i - 1 to tap i, taps beyond the ends are 0.
+		const int K = pp->psf_size, W = K + 3;
 		auto cdfOf = [&](const std::vector<float>& t)
 		{
 			std::vector<float4> out(static_cast<size_t>(pp->psf_num_s) * W);
 			const double step = pp->psf_k_spacing;
+			std::vector<double> value(W);
 			for (int i = 0; i < pp->psf_num_s; i++)
 			{
 				auto v = [&](int k) { return (k < 0 || k >= K) ? 0.0 : double(t[size_t(i) * K + k]); };
-				double whole = 0.0;
+				const int mid = (K + 1) / 2;
+				value[0] = value[K + 1] = value[K + 2] = 0.0;
+				for (int m = 1; m < mid; m++)
+					value[m] = value[m - 1] + 0.5 * step * (v(m - 2) + v(m - 1));
+				for (int m = K; m >= mid; m--)
+					value[m] = value[m + 1] - 0.5 * step * (v(m - 1) + v(m));
 				for (int k = 0; k < K; k++)
-					whole += step * v(k);
-				double acc = 0.0;
+					value[K + 2] += step * v(k);
+				double most = 0.0;
+				for (const double x : value)
+					most = std::max(most, std::fabs(x));
+				const double unit = most > 0.0 && std::isfinite(most) ?
+				                        std::ldexp(1.0, std::ilogb(most) - 21) :
+				                        1.0;
 				for (int m = 0; m < W; m++)
 				{
-					if (m == (K + 1) / 2)
+					float first = static_cast<float>(std::nearbyint(value[m] / unit) * unit);
+					float rest = static_cast<float>(value[m] - first);
+					if (!std::isfinite(rest))
 					{
-						// From the centre tap on, minus what is left of it.
-						acc = 0.0;
-						for (int k = m; k <= K; k++)
-							acc -= 0.5 * step * (v(k - 1) + v(k));
+						first = static_cast<float>(value[m]);
+						rest = 0.f;
 					}
 					out[size_t(i) * W + m] =
-					    make_float4(static_cast<float>(acc), static_cast<float>(step * v(m - 1)),
-					                static_cast<float>(0.5 * step * (v(m) - v(m - 1))), 0.f);
-					acc += 0.5 * step * (v(m - 1) + v(m));
+					    make_float4(first, static_cast<float>(step * v(m - 1)),
+					                static_cast<float>(0.5 * step * (v(m) - v(m - 1))), rest);
 				}
-				out[size_t(i) * W].w = static_cast<float>(whole);
 			}
 			return out;
 		};
