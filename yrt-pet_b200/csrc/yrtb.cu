@@ -535,21 +535,22 @@ __device__ __forceinline__ float forwardEvent(const KParams& P,
 			return __ldg(img + o);
 		}
 	};
+	// Compensated sum of the ray's products.
+	auto add = [&](float w, float q)
+	{
+		const float y = __fmaf_rn(w, q, -comp);
+		const float t = ray + y;
+		comp = (t - ray) - y;
+		ray = t;
+	};
 	auto visit = [&](int o, float w)
 	{
 		if constexpr (TRACK)
 			mw = fmaxf(mw, fabsf(w));
 		if constexpr (COMP)
-		{
-			const float y = __fmaf_rn(w, fetch(o), -comp);
-			const float t = ray + y;
-			comp = (t - ray) - y;
-			ray = t;
-		}
+			add(w, fetch(o));
 		else
-		{
 			ray += w * fetch(o);
-		}
 	};
 	auto endRay = [&]
 	{
@@ -563,25 +564,21 @@ __device__ __forceinline__ float forwardEvent(const KParams& P,
 		auto quad = [&](int o, float4 w)
 		{
 			const float4 q = __ldg(reinterpret_cast<const float4*>(img + o));
-			float c = w.x != 0.f ? w.x * q.x : 0.f;
-			c = w.y != 0.f ? __fmaf_rn(w.y, q.y, c) : c;
-			c = w.z != 0.f ? __fmaf_rn(w.z, q.z, c) : c;
-			c = w.w != 0.f ? __fmaf_rn(w.w, q.w, c) : c;
-			const float y = c - comp;
-			const float t = ray + y;
-			comp = (t - ray) - y;
-			ray = t;
+			add(w.x, w.x != 0.f ? q.x : 0.f);
+			add(w.y, w.y != 0.f ? q.y : 0.f);
+			add(w.z, w.z != 0.f ? q.z : 0.f);
+			add(w.w, w.w != 0.f ? q.w : 0.f);
 		};
 		projectEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2, tofv, rid, true, quad, endRay, part,
 		                              parts);
 	}
 	else if constexpr (KIND == K_DD_PSF && COMP)
 	{
-		// A column's products are summed before they enter the compensated
-		// sum: its reads are in flight together.
+		// A column's reads are in flight together; each product enters the
+		// compensated sum.
 		auto column = [&](int o, int stride, float w, const float(&zq)[kDDZ], unsigned mask)
 		{
-			float q[kDDZ], c = 0.f;
+			float q[kDDZ];
 #pragma unroll
 			for (int j = 0; j < kDDZ; j++)
 				q[j] = (mask & (1u << j)) ? __ldg(img + o + j * stride) : 0.f;
@@ -590,15 +587,11 @@ __device__ __forceinline__ float forwardEvent(const KParams& P,
 			{
 				if (mask & (1u << j))
 				{
-					c = __fmaf_rn(zq[j], q[j], c);
+					add(w * zq[j], q[j]);
 					if constexpr (TRACK)
 						mw = fmaxf(mw, fabsf(w * zq[j]));
 				}
 			}
-			const float y = __fmaf_rn(w, c, -comp);
-			const float t = ray + y;
-			comp = (t - ray) - y;
-			ray = t;
 		};
 		projectEvent<KIND, TOF, COMP>(P, p1, p2, n1, n2, tofv, rid, true, column, endRay, part,
 		                              parts);
