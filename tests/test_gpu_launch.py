@@ -304,22 +304,24 @@ def test_small_launches_equal_the_set_shape(precision, tof, n):
     x = torch.from_numpy(rng.random(ip.shape, np.float32)).cuda()
     y = torch.from_numpy(f32(0, 1)).cuda()
     out = {}
-    for shape in ("default", "set"):
+    # The default shape, the EM pass's batched form with its float4, pair and
+    # scalar reductions, and float4 gathers with staged reductions, which neither
+    # batch nor walk in lock step.
+    for shape in (None, (256, 2), (128, 8), (128, 0), (256, 5)):
         p = yrt.DeviceProjector(sc, ip, pp)
-        if shape == "set":
-            # Float4 gathers and staged reductions: neither batches nor
-            # lock step.
-            p.set_launch(256, 1, 3, vector_groups=5)
+        if shape:
+            p.set_launch(shape[0], 1, 3, vector_groups=shape[1])
         fwd = p.forward(x, ev, out=torch.full((m,), -3.0, device="cuda"), rng=r)
         bwd = p.backward(y, ev, rng=r)
         em, model = torch.zeros_like(x), torch.full((m,), -3.0, device="cuda")
         p.em_step(x, em, ev, rng=r, global_scale=0.7, model=model)
         out[shape] = (fwd, model, bwd, em, p.take_event_errors())
-    a, b = out["default"], out["set"]
-    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
-    assert a[4] == b[4]
-    for i in (2, 3):  # the same terms, added in another order
-        assert rel_l2(a[i].cpu().numpy(), b[i].cpu().numpy()) < 2 * n ** 0.5 * 2.0 ** -24
+    b = out.pop((256, 5))
+    for a in out.values():
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+        assert a[4] == b[4]
+        for i in (2, 3):  # the same terms, added in another order
+            assert rel_l2(a[i].cpu().numpy(), b[i].cpu().numpy()) < 2 * n ** 0.5 * 2.0 ** -24
 
 
 def launched_blocks(call):

@@ -114,15 +114,20 @@ def test_operator_projector_device_reference_signatures(kind):
 
 
 # Subsets of one or many phi, a subset with fewer phi than the others, both
-# precisions and every projector; the lists of crystal pairs are the oracle.
-@pytest.mark.parametrize("projector,rays", [("S", 1), ("S", 3), ("DD", 1)])
+# precisions and every projector (DD with a kernel that is not symmetric); the
+# lists of crystal pairs are the oracle.  Values up to 1, and a large one on a
+# bin that misses the grid, which must not set the scale of the others.
+@pytest.mark.parametrize("projector,rays", [("S", 1), ("S", 3), ("DD", 1), ("DD+PSF", 1)])
 @pytest.mark.parametrize("comp,det", [(False, False), (True, False), (False, True), (True, True)])
 @pytest.mark.parametrize("subsets,subset", [(1, 0), (7, 6), (32, 31)])
 def test_histogram_bins_equal_crystal_pairs(projector, rays, comp, det, subsets, subset):
     sc = yrt.Scanner("t", 40, 4, 4, 10, 100, 32, 6, 1, 4, 3, 1)
     ip = yrt.ImageParams(21, 18, 10, 105.0, 90.0, 40.0)
     pp = yrt.ProjectorParams(sc)
-    pp.setProjector(projector)
+    pp.setProjector(projector[:2] if projector != "S" else "S")
+    if projector == "DD+PSF":
+        k = np.roll(np.exp(-0.5 * ((np.arange(17) - 8) * 0.6 / 1.7) ** 2), 1)
+        pp.setProjPsf(30.0, 0.6, np.stack([k, k[::-1] ** 2]).astype(np.float32))
     pp.numRays = rays
     pp.precision = L.YRTB_COMPENSATED if comp else L.YRTB_MIRROR
     pp.deterministic = det
@@ -137,7 +142,11 @@ def test_histogram_bins_equal_crystal_pairs(projector, rays, comp, det, subsets,
     idx = torch.from_numpy(bins).cuda()
     want = torch.full((h.histoSize,), -7.0, device="cuda")
     want[idx] = p.forward(x, ev)
+    miss = torch.nonzero(want[idx] == 0).reshape(-1)
+    if miss.numel():
+        w[idx[miss[0]]] = 1e12
     want_img = p.backward(w[idx].contiguous(), ev)
+    assert float(want_img.max()) > 0
     op = yrt.OperatorProjectorDevice.create(pp, it, img_params=ip)
     got = yrt.ProjectionList(h)
     got.values = torch.full((h.histoSize,), -7.0, device="cuda")
