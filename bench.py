@@ -805,12 +805,17 @@ def main():
                        "reconstruction of 3 OSEM iterations x 10 subsets, D2H "
                        "image"}
 
+    # Float4 gathers, staged reductions, tiled images and split rays take the
+    # kernel that walks one crossing at a time.
+    batched = (not tiled and launch["threads_per_lor"] == 1 and
+               not launch["vector_groups"] & 5)
     peak, peak_kind = measured_peak_hbm()
     achieved = alg_bytes_iter / SUBSETS / (em_ms * 1e-3) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": None,
-                "kernel": "k_events<OP_EM, K_SIDDON, TOF> (fused fwd->ratio->bwd)",
+                "kernel": ("k_events_batch<OP_EM, TOF>" if batched else
+                           "k_events<OP_EM, K_SIDDON, TOF>") + " (fused fwd->ratio->bwd)",
                 "alg_bytes_per_launch": alg_bytes_iter / SUBSETS,
                 "mean_crossings_per_event": n_vox_total / ev.count,
                 "em_kernel_ms_per_launch": em_ms}

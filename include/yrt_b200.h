@@ -177,7 +177,9 @@ void yrtb_projector_destroy(yrtb_projector* h);
  * No reference counterpart: the reference launches one thread per event in
  * 256-thread blocks (GPUBatchSetup, include/yrt-pet/utils/GPUTypes.cuh:17-55)
  * on events in file order.  Default: {256, 1, 3, order, 1, 2}, the order
- * YRTB_ORDER_SPATIAL for single-ray Siddon with TOF, else YRTB_ORDER_LOR. */
+ * YRTB_ORDER_SPATIAL for single-ray Siddon with TOF, else YRTB_ORDER_LOR.
+ * Until a configuration is set or tuned, single-ray Siddon forward projections
+ * and launches of few events run in one-warp blocks. */
 #define YRTB_ORDER_LOR 0      /* inside a ray-length bucket: by LOR (Histogram3D bin), then TOF */
 #define YRTB_ORDER_SPATIAL 1  /* inside a ray-length bucket: by direction sector (16 azimuthal x
                                  2 axial), then the Morton code of the TOF kernel centre (the
@@ -209,9 +211,11 @@ typedef struct
 	                         bit 3: pairs of voxels sent as one red.global.add.v2.f32 (bits 1
 	                         and 2 win over it).  Multi-ray walks use bits 1 and 3 (each ray's
 	                         group or pair sent at the end of the ray; default 8 with one
-	                         lane per ray, else 2).  Images must be
-	                         16-byte aligned with a multiple of 4 voxels per frame, else
-	                         scalar accesses are used */
+	                         lane per ray, else 2).  Images must be 16-byte aligned and,
+	                         with several frames, have a multiple of 4 voxels per frame,
+	                         else scalar accesses are used; bit 0 also needs a multiple of
+	                         4 voxels of a single frame (the reductions send a last part
+	                         of a group voxel by voxel) */
 } yrtb_launch_config;
 
 yrtb_status yrtb_projector_set_launch(yrtb_projector* h,
